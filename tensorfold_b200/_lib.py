@@ -10,6 +10,8 @@ import os
 
 LIB_PATH = Path(os.environ.get("TENSORFOLD_B200_LIB") or Path(__file__).resolve().parent / "libtensorfold_b200.so")
 
+NATIVE_PATH = Path(__file__).resolve().parent / "_native.so"
+
 _vp, _i32, _i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
 
 # name -> (restype, argtypes); mirrors include/tensorfold_b200.h
@@ -100,17 +102,28 @@ def ensure_device(index: int) -> None:
         _ready.add(index)
 
 
-def stream_of(t) -> int:
-    import torch
+@lru_cache(maxsize=1)
+def native():
+    """The host path as an extension module (``csrc/native.cpp``): whole wrappers for the calls an engine issues per
+    layer, and one thunk per C-ABI entry, ``native().tf_x(what, ...)``, that takes tensors where the entry takes pointers
+    and raises like ``check``."""
 
-    if not t.is_cuda:
-        raise ValueError("operands must live on a CUDA device: this path has no CPU implementation")
-    ensure_device(t.device.index)
-    if t.device.index != torch.cuda.current_device():
-        # the entry points take per-device state (error word, SM count, built-in scratch) from the CURRENT device
-        raise ValueError(f"operands live on cuda:{t.device.index} but cuda:{torch.cuda.current_device()} is current: "
-                         "call under torch.cuda.device(tensor.device)")
-    return torch.cuda.current_stream(t.device).cuda_stream
+    lib()
+    if not NATIVE_PATH.exists():
+        raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m tensorfold_b200.build`")
+    import torch                            # noqa: F401  (its libraries must be loaded before the module's)
+
+    from . import _native
+
+    _native.bind(str(LIB_PATH), ensure_device)
+    return _native
+
+
+def stream_of(t) -> int:
+    """The current stream of the tensor's device, which must be the current device (it holds the error word, the SM count
+    and the built-in scratch the entry points use)."""
+
+    return native().stream_of(t)
 
 
 def device_error(t) -> int:

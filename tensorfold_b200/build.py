@@ -1,4 +1,5 @@
-"""Builds ``libtensorfold_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds ``libtensorfold_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU), and beside it
+``_native.so``, the host path as a CPython extension over torch's C++ tensors (``csrc/native.cpp``, the C++ compiler alone).
 
     python -m tensorfold_b200.build [--force]
 
@@ -11,6 +12,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +20,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "libtensorfold_b200.so"
+NATIVE = HERE / "_native.so"
 BITS = (2, 3, 4, 5, 6, 8)
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--threads", "2"]
@@ -46,14 +49,36 @@ def _compile(unit) -> str:
     return obj.name
 
 
+def _native() -> str:
+    """Compiles the extension module against the torch that will load it."""
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    heads = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+             Path(sysconfig.get_paths()["include"])]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *(f"-I{h}" for h in heads), str(CSRC / "native.cpp"), "-o", str(NATIVE), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda",
+           "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ldl"]
+    done = subprocess.run(cmd, capture_output=True, text=True)
+    if done.returncode:
+        raise RuntimeError(f"g++ failed for native.cpp:\n{done.stdout}\n{done.stderr}")
+    return NATIVE.name
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(exist_ok=True)
     heads = _newest_header()
     stale = [u for u in _units()
              if force or not u[1].exists() or u[1].stat().st_mtime < max(u[0].stat().st_mtime, heads)]
-    if stale:
-        with ThreadPoolExecutor(max_workers=min(len(stale), os.cpu_count() or 4)) as pool:
-            for name in pool.map(_compile, stale):
+    source = CSRC / "native.cpp"
+    native = force or not NATIVE.exists() or NATIVE.stat().st_mtime < max(
+        source.stat().st_mtime, (HERE.parent / "include" / "tensorfold_b200.h").stat().st_mtime)
+    jobs = ([_native] if native else []) + [lambda u=u: _compile(u) for u in stale]
+    if jobs:
+        with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as pool:
+            for name in pool.map(lambda job: job(), jobs):
                 if verbose:
                     print("compiled", name)
     objs = [str(u[1]) for u in _units()]

@@ -145,9 +145,8 @@ def route(picks: torch.Tensor, plan: Plan) -> None:
     if picks.dtype != torch.int32 or not picks.is_contiguous():
         raise ValueError("picks must be contiguous int32")
     stream = _lib.stream_of(picks)
-    _lib.check(_lib.lib().tf_moe_plan(picks.data_ptr(), rows * slots, plan.experts, plan.tile, plan.members.data_ptr(),
-                                      plan.items.data_ptr(), plan.counts.data_ptr(), plan.rank.data_ptr(),
-                                      plan.hist.data_ptr(), plan.items.shape[0], stream), "route")
+    _lib.native().tf_moe_plan("route", picks, rows * slots, plan.experts, plan.tile, plan.members, plan.items, plan.counts,
+                              plan.rank, plan.hist, plan.items.shape[0], stream)
 
 
 def _grouped(x, slots, table, n, k, ex, plan, out, rows, epi, limit):
@@ -168,15 +167,13 @@ def _grouped(x, slots, table, n, k, ex, plan, out, rows, epi, limit):
         pairs = plan.members.shape[0]
         if plan.sorted is None or plan.sorted.numel() < pairs * k:
             plan.sorted = torch.empty((pairs * max(k, ex.dims, ex.width),), dtype=torch.bfloat16, device=x.device)
-        _lib.check(_lib.lib().tf_moe_experts_prefill(
-            x.data_ptr(), x.stride(0), slots, table.data_ptr(), table.stride(0), table.shape[0], n, k, ex.gs, plan.items.data_ptr(),
-            plan.counts.data_ptr(), plan.members.data_ptr(), rows * plan.slots, items, plan.sorted.data_ptr(), out.data_ptr(),
-            out.stride(0), int(out.dtype == torch.float32), epi, float(limit), stream), "experts (prefill)")
+        _lib.native().tf_moe_experts_prefill(
+            "experts (prefill)", x, x.stride(0), slots, table, table.stride(0), table.shape[0], n, k, ex.gs, plan.items, plan.counts,
+            plan.members, rows * plan.slots, items, plan.sorted, out, out.stride(0), out.dtype == torch.float32, epi, limit, stream)
         return
-    _lib.check(_lib.lib().tf_moe_experts(
-        x.data_ptr(), x.stride(0), slots, table.data_ptr(), table.stride(0), table.shape[0], n, k, ex.gs, plan.items.data_ptr(),
-        plan.counts.data_ptr(), plan.members.data_ptr(), items, plan.tile, out.data_ptr(), out.stride(0),
-        int(out.dtype == torch.float32), epi, float(limit), stream), "experts")
+    _lib.native().tf_moe_experts(
+        "experts", x, x.stride(0), slots, table, table.stride(0), table.shape[0], n, k, ex.gs, plan.items, plan.counts, plan.members,
+        items, plan.tile, out, out.stride(0), out.dtype == torch.float32, epi, limit, stream)
 
 
 def gate_up(x: torch.Tensor, ex: Experts, plan: Plan, out: torch.Tensor, rows: int) -> None:

@@ -108,7 +108,6 @@ def embed(ids, q):
     out = torch.empty((ids.shape[0], k), dtype=torch.bfloat16, device=ids.device)
     for a in range(0, ids.shape[0], 65535):
         part = ids[a:a + 65535]
-        _lib.check(_lib.lib().tf_affine_rows(part.data_ptr(), int(ids.dtype == torch.int64), part.shape[0], q.weight.data_ptr(),
-                                             q.scales.data_ptr(), q.biases.data_ptr(), meta, n, k, q.bits, q.gs,
-                                             out[a:a + 65535].data_ptr(), 0, stream), "embed")
+        _lib.native().tf_affine_rows("embed", part, ids.dtype == torch.int64, part.shape[0], q.weight, q.scales, q.biases, meta, n,
+                                     k, q.bits, q.gs, out[a:a + 65535], 0, stream)
     return out

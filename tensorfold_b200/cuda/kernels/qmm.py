@@ -6,9 +6,9 @@ argument meaning and errors; the arithmetic runs in ``libtensorfold_b200.so``.
 
 from __future__ import annotations
 
-import ctypes
 import os
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -16,6 +16,20 @@ from ... import _lib
 
 BITS = (2, 3, 4, 5, 6, 8)
 GROUPS = (32, 64, 128)
+
+
+@lru_cache(maxsize=1)
+def _native():
+    """The extension module, told the two rules that stay here: K slices of a shape, and a stream's scratch."""
+
+    module = _lib.native()
+    module.hooks(default_split, _scratch_for)
+    return module
+
+
+@lru_cache(maxsize=None)
+def _unit_words(bits: int, gs: int) -> int:
+    return _lib.lib().tf_unit_words(bits, gs)
 
 
 @dataclass
@@ -53,11 +67,8 @@ def pack(weight: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor, gs: i
         raise ValueError(f"pack: words {tuple(weight.shape)} do not match scales {tuple(scales.shape)} at {bits} bits")
     stream = _lib.stream_of(weight)
     weight, scales, biases = weight.contiguous(), scales.contiguous(), biases.contiguous()
-    lib = _lib.lib()
-    unit = lib.tf_unit_words(bits, gs)
-    out = torch.empty((-(-n // 128), k // gs, unit), dtype=torch.int32, device=weight.device)
-    _lib.check(lib.tf_pack(weight.data_ptr(), scales.data_ptr(), biases.data_ptr(), n, k, bits, gs, out.data_ptr(),
-                           stream), "pack")
+    out = torch.empty((-(-n // 128), k // gs, _unit_words(bits, gs)), dtype=torch.int32, device=weight.device)
+    _native().tf_pack("pack", weight, scales, biases, n, k, bits, gs, out, stream)
     return Q4(out, None, None, n, k, gs, bits)
 
 
@@ -70,8 +81,7 @@ def unpack(q: Q4, chunk: int = 64) -> tuple[torch.Tensor, torch.Tensor, torch.Te
     scales = torch.empty((q.n, q.k // q.gs), dtype=torch.bfloat16, device=dev)
     biases = torch.empty_like(scales)
     tiled = q.weight if q.weight.is_contiguous() else q.weight.contiguous()
-    _lib.check(_lib.lib().tf_unpack(tiled.data_ptr(), q.n, q.k, q.bits, q.gs, words.data_ptr(), scales.data_ptr(),
-                                    biases.data_ptr(), stream), "unpack")
+    _native().tf_unpack("unpack", tiled, q.n, q.k, q.bits, q.gs, words, scales, biases, stream)
     return words, scales, biases
 
 
@@ -127,18 +137,8 @@ def group_sums(x: torch.Tensor, gs: int = 64) -> torch.Tensor:
     stream = _lib.stream_of(x)
     m, k = x.shape
     xs = torch.empty((m, k // gs), dtype=torch.float32, device=x.device)
-    _lib.check(_lib.lib().tf_group_sums(x.data_ptr(), x.stride(0), m, k, gs, xs.data_ptr(), stream), "group_sums")
+    _native().tf_group_sums("group_sums", x, x.stride(0), m, k, gs, xs, stream)
     return xs
-
-
-def _rows(x: torch.Tensor, k: int, who: str) -> torch.Tensor:
-    if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != k:
-        raise ValueError(f"{who}: x must be (M, {k}) bf16")
-    if x.shape[0] < 1:
-        raise ValueError(f"{who}: x needs at least one row")
-    if x.stride(1) != 1 or (x.shape[0] > 1 and x.stride(0) % 8) or x.data_ptr() % 16:
-        x = x.clone(memory_format=torch.contiguous_format)     # bulk copies read rows in 16-byte pieces
-    return x
 
 
 def matmul(x: torch.Tensor, q: Q4, xs: torch.Tensor | None = None, *, sk: int | None = None, f32: bool = False,
@@ -149,65 +149,31 @@ def matmul(x: torch.Tensor, q: Q4, xs: torch.Tensor | None = None, *, sk: int | 
     ``pdl`` (not in the reference) launches with programmatic stream serialisation so the weight prefetch of this call
     overlaps the end of the previous kernel in the stream."""
 
-    x = _rows(x, q.k, "matmul")
-    m = x.shape[0]
-    stream = _lib.stream_of(x)
-    if q.weight.device != x.device:
-        raise ValueError("matmul: x and the weight must share a CUDA device")
-    kg = q.k // q.gs
-    if xs is not None and (xs.dtype != torch.float32 or xs.shape != (m, kg) or not xs.is_contiguous()):
-        raise ValueError(f"matmul: xs must be contiguous ({m}, {kg}) fp32")
-    sk = sk or default_split(q.n, q.k, q.gs)
-    if sk < 1 or sk > kg:
-        raise ValueError("matmul: 1 to K / gs slices (a slice holds one group at least)")
-    slices = sk > 1 and not reduce
-    if out is None:
-        if not slices:
-            out = torch.empty((m, q.n), dtype=torch.float32 if f32 else torch.bfloat16, device=x.device)
-    elif out.shape != (m, q.n) or out.dtype != (torch.float32 if f32 else torch.bfloat16) or out.stride(1) != 1:
-        raise ValueError("matmul: out must be (M, n) of the requested dtype with unit-stride rows")
-    if sk > 1 and (not reduce or sk > 8):
-        if part is None:
-            part = torch.empty((sk, m, q.n), dtype=torch.float32, device=x.device)
-        elif part.dtype != torch.float32 or not part.is_contiguous() or part.numel() < sk * m * q.n:
-            raise ValueError("matmul: part must hold (SK, M, n) fp32")
-    if q.weight.dim() != 3 or q.weight.stride(2) != 1 or q.weight.stride(1) != q.weight.shape[2]:
-        raise ValueError("matmul: the tiled weight may be sliced by super-blocks of 128 columns only")
-    if STREAM and m <= STREAM_ROWS and part is None and (reduce or sk == 1):
-        return matmul_set(x, [q], xs, sks=[sk], f32=f32, outs=[out], pdl=pdl)[0]     # same bits, persistent launch
-    _lib.check(_lib.lib().tf_qmm(
-        x.data_ptr(), x.stride(0), m, xs.data_ptr() if xs is not None else None, q.weight.data_ptr(),
-        q.weight.stride(0), q.n, q.k, q.bits, q.gs, sk, out.data_ptr() if out is not None else None,
-        out.stride(0) if out is not None else 0, int(f32), part.data_ptr() if part is not None else None,
-        int(reduce), int(pdl), stream), "matmul")
-    if sk == 1 or reduce:
-        return out
-    return part.reshape(-1)[:sk * m * q.n].view(sk, m, q.n)
+    return _native().matmul(x, q, xs, sk, f32, out, part, reduce, pdl, STREAM)
 
 
 STREAM = os.environ.get("TENSORFOLD_B200_STREAM", "1") != "0"      # decode windows run the persistent kernel (same bits)
-STREAM_ROWS = 16
-SET_MAX = 4
 SCRATCH_BYTES = 16 << 20          # one scratch area: room for a gate/up set of 17408 rows each in 4 K slices
 SCRATCH_AREAS = 4                 # areas made on a device's first call: the calling stream's and three side streams'
 _set_scratch: dict = {}           # (device index, stream) -> the stream's scratch area
 _free_areas: dict = {}            # device index -> areas not yet handed to a stream
 
 
-def _scratch_for(device: torch.device, stream: int, need: int) -> torch.Tensor:
-    """The scratch area of (device, stream) where the K slices of a set meet: zeroed once, left zero by every call.
+def _scratch_for(index: int, stream: int, need: int) -> torch.Tensor:
+    """The scratch area of (device index, stream) where the K slices of a set meet: zeroed once, left zero by every call.
+    The extension asks for it when it has not seen the stream, or the area it knows is too small.
 
     Areas are made eagerly (four on a device's first call, more when a fifth stream shows up or a set needs more room)
     and only handed out during a stream capture: a graph must not own memory that later calls use, so a capture that
     would need a new allocation is refused with a message saying which eager call to make first."""
 
-    key = (device.index, stream)
+    device, key = torch.device("cuda", index), (index, stream)
     buf = _set_scratch.get(key)
     if buf is not None and buf.numel() >= need:
         return buf
     capturing = torch.cuda.is_current_stream_capturing()
-    free = _free_areas.setdefault(device.index, [])
-    if not free and not capturing and not any(k[0] == device.index for k in _set_scratch):
+    free = _free_areas.setdefault(index, [])
+    if not free and not capturing and not any(k[0] == index for k in _set_scratch):
         free.extend(torch.zeros((SCRATCH_BYTES,), dtype=torch.uint8, device=device) for _ in range(SCRATCH_AREAS))
     fits = [i for i, area in enumerate(free) if area.numel() >= need]
     if buf is None and fits:
@@ -226,6 +192,7 @@ def reset_scratch() -> None:
 
     _set_scratch.clear()
     _free_areas.clear()
+    _native().forget_scratch()
 
 
 def matmul_set(x: torch.Tensor, qs, xs: torch.Tensor | None = None, *, sks=None, f32: bool = False, outs=None,
@@ -234,48 +201,7 @@ def matmul_set(x: torch.Tensor, qs, xs: torch.Tensor | None = None, *, sks=None,
     the bits ``matmul(x, q, sk=sk)`` gives.  1 to 16 rows, up to 4 weights of one format and K.  Not in the reference,
     whose engines issue these as separate calls (families/qwen3_5/cuda/qmm_fast.py:49-64)."""
 
-    qs = list(qs)
-    if not 1 <= len(qs) <= SET_MAX:
-        raise ValueError(f"matmul_set: 1 to {SET_MAX} weights a set")
-    q0 = qs[0]
-    if any((q.k, q.gs, q.bits) != (q0.k, q0.gs, q0.bits) for q in qs):
-        raise ValueError("matmul_set: the weights of a set share K, group and bit width")
-    x = _rows(x, q0.k, "matmul_set")
-    m = x.shape[0]
-    if m > STREAM_ROWS:
-        raise ValueError(f"matmul_set: at most {STREAM_ROWS} rows (use matmul for larger windows)")
-    stream = _lib.stream_of(x)
-    kg = q0.k // q0.gs
-    if xs is not None and (xs.dtype != torch.float32 or xs.shape != (m, kg) or not xs.is_contiguous()):
-        raise ValueError(f"matmul_set: xs must be contiguous ({m}, {kg}) fp32")
-    sks = [sk or default_split(q.n, q.k, q.gs) for q, sk in zip(qs, sks or [None] * len(qs))]
-    outs = list(outs) if outs is not None else [None] * len(qs)
-    dtype = torch.float32 if f32 else torch.bfloat16
-    for i, q in enumerate(qs):
-        if q.weight.device != x.device:
-            raise ValueError("matmul_set: x and the weights must share a CUDA device")
-        if sks[i] < 1 or sks[i] > kg:
-            raise ValueError("matmul_set: 1 to K / gs slices (a slice holds one group at least)")
-        if q.weight.dim() != 3 or q.weight.stride(2) != 1 or q.weight.stride(1) != q.weight.shape[2]:
-            raise ValueError("matmul_set: the tiled weight may be sliced by super-blocks of 128 columns only")
-        if outs[i] is None:
-            outs[i] = torch.empty((m, q.n), dtype=dtype, device=x.device)
-        elif outs[i].shape != (m, q.n) or outs[i].dtype != dtype or outs[i].stride(1) != 1:
-            raise ValueError("matmul_set: out must be (M, n) of the requested dtype with unit-stride rows")
-    count = len(qs)
-    ints, longs, ptrs = ctypes.c_int * count, ctypes.c_int64 * count, ctypes.c_void_p * count
-    n_arr, sk_arr = ints(*[q.n for q in qs]), ints(*sks)
-    lib = _lib.lib()
-    need = lib.tf_qmm_set_scratch_bytes(count, n_arr, sk_arr)
-    if need < 0:
-        raise ValueError("matmul_set: bad shapes")
-    scratch = _scratch_for(x.device, stream, need)
-    _lib.check(lib.tf_qmm_set(
-        x.data_ptr(), x.stride(0), m, xs.data_ptr() if xs is not None else None, q0.k, q0.bits, q0.gs, count,
-        ptrs(*[q.weight.data_ptr() for q in qs]), longs(*[q.weight.stride(0) for q in qs]), n_arr, sk_arr,
-        ptrs(*[o.data_ptr() for o in outs]), longs(*[o.stride(0) for o in outs]), int(f32), scratch.data_ptr(),
-        scratch.numel(), int(pdl), stream), "matmul_set")
-    return outs
+    return _native().matmul_set(x, qs, xs, sks, f32, outs, pdl)
 
 
 def prefill_matmul(x: torch.Tensor, q: Q4, *, f32: bool = False, tile: int = 0,
@@ -284,18 +210,9 @@ def prefill_matmul(x: torch.Tensor, q: Q4, *, f32: bool = False, tile: int = 0,
     same bits, not decode's.  ``tile`` is accepted for signature parity (cuda/kernels/qmm.py:160) and unused.  Formats
     the tcgen05 kernel does not take (other widths, groups of 128, K not a multiple of 64) run through ``matmul``."""
 
-    x = _rows(x, q.k, "prefill_matmul")
     if q.bits != 4 or q.gs not in (32, 64) or q.k % 64:
         return matmul(x, q, f32=f32, out=out)
-    m = x.shape[0]
-    stream = _lib.stream_of(x)
-    if out is None:
-        out = torch.empty((m, q.n), dtype=torch.float32 if f32 else torch.bfloat16, device=x.device)
-    elif out.shape != (m, q.n) or out.dtype != (torch.float32 if f32 else torch.bfloat16) or out.stride(1) != 1:
-        raise ValueError("prefill_matmul: out must be (M, n) of the requested dtype with unit-stride rows")
-    _lib.check(_lib.lib().tf_qmm_prefill(x.data_ptr(), x.stride(0), m, q.weight.data_ptr(), q.weight.stride(0), q.n, q.k, q.gs,
-                                         out.data_ptr(), out.stride(0), int(f32), stream), "prefill_matmul")
-    return out
+    return _native().prefill_matmul(x, q, f32, out)
 
 
 _side_streams: dict = {}
@@ -346,9 +263,8 @@ def pack_pair(gate: tuple, up: tuple, gs: int, bits: int = 4) -> Q4:
         raise ValueError("pack_pair: rows in whole 16-row tiles, bf16 scales and biases")
     stream = _lib.stream_of(wg)
     ts = [t.contiguous() for t in (wg, sg, bg, wu, su, bu)]
-    lib = _lib.lib()
-    out = torch.empty((-(-2 * n // 128), k // gs, lib.tf_unit_words(bits, gs)), dtype=torch.int32, device=wg.device)
-    _lib.check(lib.tf_pack_pair(*[t.data_ptr() for t in ts], n, k, bits, gs, out.data_ptr(), stream), "pack_pair")
+    out = torch.empty((-(-2 * n // 128), k // gs, _unit_words(bits, gs)), dtype=torch.int32, device=wg.device)
+    _native().tf_pack_pair("pack_pair", *ts, n, k, bits, gs, out, stream)
     return Q4(out, None, None, 2 * n, k, gs, bits)
 
 
@@ -357,22 +273,6 @@ def matmul_act(x: torch.Tensor, q: Q4, *, act: str = "swiglu", limit: float = 0.
     """Projection with the experts' activation epilogue, dense form: ``act="swiglu"`` on a ``pack_pair`` weight gives
     bf16(bf16(silu(bf16 gate)) * bf16 up) as (M, n / 2); ``act="relu2"`` gives bf16(relu(bf16 v)^2) as (M, n)."""
 
-    x = _rows(x, q.k, "matmul_act")
     if act not in ("swiglu", "relu2"):
         raise ValueError("matmul_act: act is 'swiglu' or 'relu2'")
-    m = x.shape[0]
-    stream = _lib.stream_of(x)
-    ncols = q.n // 2 if act == "swiglu" else q.n
-    if out is None:
-        out = torch.empty((m, ncols), dtype=torch.bfloat16, device=x.device)
-    elif out.shape != (m, ncols) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
-        raise ValueError("matmul_act: out must be (M, columns) bf16 with unit-stride rows")
-    if prefill and q.bits == 4 and q.gs in (32, 64):          # the prefill arithmetic (weights rounded once to bf16)
-        _lib.check(_lib.lib().tf_qmm_prefill_act(x.data_ptr(), x.stride(0), m, q.weight.data_ptr(), q.weight.stride(0), q.n, q.k,
-                                                 q.gs, out.data_ptr(), out.stride(0), 0, 2 if act == "swiglu" else 1,
-                                                 float(limit), stream), "matmul_act (prefill)")
-        return out
-    _lib.check(_lib.lib().tf_qmm_act(x.data_ptr(), x.stride(0), m, q.weight.data_ptr(), q.weight.stride(0), q.n, q.k, q.bits,
-                                     q.gs, out.data_ptr(), out.stride(0), 2 if act == "swiglu" else 1, float(limit), int(pdl),
-                                     stream), "matmul_act")
-    return out
+    return _native().matmul_act(x, q, act == "swiglu", limit, out, pdl, prefill)

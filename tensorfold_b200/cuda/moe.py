@@ -26,8 +26,8 @@ def router(x: torch.Tensor, rows: torch.Tensor, out: torch.Tensor | None = None,
     if out is None:
         out = torch.empty((m, ne), dtype=torch.float32, device=x.device)
     stream = _lib.stream_of(x)
-    fn = _lib.lib().tf_moe_router_tiles if prefill else _lib.lib().tf_moe_router
-    _lib.check(fn(x.data_ptr(), x.stride(0), m, d, rows.data_ptr(), ne, out.data_ptr(), out.stride(0), stream), "router")
+    fn = _lib.native().tf_moe_router_tiles if prefill else _lib.native().tf_moe_router
+    fn("router", x, x.stride(0), m, d, rows, ne, out, out.stride(0), stream)
     return out
 
 
@@ -54,8 +54,7 @@ def select_rows(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts: int)
     if logits.dtype != torch.float32 or logits.stride(1) != 1 or logits.shape[1] < experts + 1:
         raise ValueError("select_rows: logits must be (R, E + 1) fp32")
     stream = _lib.stream_of(logits)
-    _lib.check(_lib.lib().tf_moe_topk(logits.data_ptr(), logits.stride(0), rows, experts, top_k, 1, buf.pick.data_ptr(),
-                                      buf.wts.data_ptr(), stream), "select_rows")
+    _lib.native().tf_moe_topk("select_rows", logits, logits.stride(0), rows, experts, top_k, 1, buf.pick, buf.wts, stream)
 
 
 def select_local_rows(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts: int, first: int, count: int) -> None:
@@ -65,8 +64,8 @@ def select_local_rows(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts
     rows = logits.shape[0]
     if logits.dtype != torch.float32 or logits.stride(1) != 1 or logits.shape[1] < experts:
         raise ValueError("select_local_rows: logits must be (R, E) fp32")
-    _lib.check(_lib.lib().tf_moe_topk_local(logits.data_ptr(), logits.stride(0), rows, experts, top_k, 1, first, count,
-                                            buf.pick.data_ptr(), buf.wts.data_ptr(), _lib.stream_of(logits)), "select_local_rows")
+    _lib.native().tf_moe_topk_local("select_local_rows", logits, logits.stride(0), rows, experts, top_k, 1, first, count, buf.pick,
+                                    buf.wts, _lib.stream_of(logits))
 
 
 def select(logits: torch.Tensor, buf: MoEBuffers, top_k: int, experts: int) -> None:
@@ -130,8 +129,7 @@ def combine(y: torch.Tensor, wts: torch.Tensor, out: torch.Tensor | None = None)
     elif out.shape != (rows, dims) or out.dtype != torch.bfloat16 or not out.is_contiguous():
         raise ValueError("combine: out must be a contiguous [R, D] bf16 tensor")
     stream = _lib.stream_of(y)
-    _lib.check(_lib.lib().tf_moe_combine(y.data_ptr(), int(y.dtype == torch.bfloat16), wts.data_ptr(), rows, slots, dims,
-                                         out.data_ptr(), stream), "combine")
+    _lib.native().tf_moe_combine("combine", y, y.dtype == torch.bfloat16, wts, rows, slots, dims, out, stream)
     return out
 
 
