@@ -1,5 +1,5 @@
 // extern "C" entry points (include/tensorfold_b200.h), argument checks, and the small kernels around the matmul:
-// load-time repack and its inverse, group sums, slice reduction.
+// group sums, slice reduction.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -72,89 +72,6 @@ int fail_moe(int code, const char* msg) { return fail(code, "%s", msg); }
 int cuda_fail_moe(cudaError_t e, const char* what) { return cuda_fail(e, what); }
 
 __device__ int g_error_word;          // set by a kernel whose bounded wait gave up; read by tf_device_error
-
-// ---------------------------------------------------------------------------------------------------------------------
-// repack: one thread per output word of the tiled tensor
-// ---------------------------------------------------------------------------------------------------------------------
-
-// With a second source (words2 != null) the packed rows interleave 16 rows of the first with 16 rows of the second
-// (gate and up projections of an expert): packed row r comes from source (r / 16) % 2, row (r / 32) * 16 + r % 16.
-__global__ void pack_kernel(const uint32_t* __restrict__ words, const uint16_t* __restrict__ scales,
-                            const uint16_t* __restrict__ biases, const uint32_t* __restrict__ words2,
-                            const uint16_t* __restrict__ scales2, const uint16_t* __restrict__ biases2, int n, int k,
-                            int bits, int gs, uint32_t* __restrict__ tiled, int64_t total) {
-  const int wpl = words_per_lane(bits, gs), unitw = unit_words(bits, gs), kg = k / gs;
-  const int64_t wpr = static_cast<int64_t>(k) * bits / 32;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int wi_unit = static_cast<int>(i % unitw);
-    const int64_t unit = i / unitw;
-    const int g = static_cast<int>(unit % kg);
-    const int64_t sb = unit / kg;
-    const int code_words = TILE_PAIRS * 32 * wpl;
-    uint32_t value;
-    if (wi_unit < code_words) {
-      const int tp = wi_unit / (32 * wpl), lane = (wi_unit / wpl) % 32, wi = wi_unit % wpl;
-      auto code = [&](int col, int kk) -> uint32_t {
-        int64_t row = sb * SB_COLS + col;
-        if (row >= n) return 0u;
-        const uint32_t* src = words;
-        if (words2 != nullptr) {
-          if ((row >> 4) & 1) src = words2;
-          row = (row >> 5) * 16 + (row & 15);
-        }
-        return stored_code(src + row * wpr, static_cast<int64_t>(g) * gs + kk, bits, wpr);
-      };
-      value = lane_word(bits, gs, tp, lane, wi, code);
-    } else {
-      const int ai = wi_unit - code_words;
-      const int tp = ai >> 5, gg = (ai >> 2) & 7, h = (ai >> 1) & 1, r8 = ai & 1;
-      int64_t row = sb * SB_COLS + 32 * tp + 16 * h + 8 * r8 + gg;
-      value = 0u;
-      if (row < n) {
-        const uint16_t *sc = scales, *bi = biases;
-        if (words2 != nullptr) {
-          if ((row >> 4) & 1) sc = scales2, bi = biases2;
-          row = (row >> 5) * 16 + (row & 15);
-        }
-        value = static_cast<uint32_t>(sc[row * kg + g]) | (static_cast<uint32_t>(bi[row * kg + g]) << 16);
-      }
-    }
-    tiled[i] = value;
-  }
-}
-
-// inverse: one thread per (row, block of 32 codes) writes `bits` words; one thread per (row, group) writes the affine pair
-__global__ void unpack_kernel(const uint32_t* __restrict__ tiled, int n, int k, int bits, int gs,
-                              uint32_t* __restrict__ words, uint16_t* __restrict__ scales, uint16_t* __restrict__ biases) {
-  const int wpl = words_per_lane(bits, gs), unitw = unit_words(bits, gs), kg = k / gs, blocks = k / 32;
-  const int64_t total = static_cast<int64_t>(n) * blocks;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t row = i / blocks;
-    const int blk = static_cast<int>(i % blocks);
-    const int64_t sb = row / SB_COLS;
-    const int c = static_cast<int>(row % SB_COLS);
-    uint32_t outw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j = 0; j < 32; ++j) {
-      const int kk_all = blk * 32 + j, g = kk_all / gs, kk = kk_all % gs;
-      const CodeLoc loc = code_loc(c, kk, gs);
-      const uint32_t* lw = tiled + (sb * kg + g) * unitw + (loc.tp * 32 + loc.lane) * wpl;
-      const uint64_t code = lane_code(bits, gs, lw, loc.p, loc.half);
-      const int bit = j * bits;
-      const uint64_t shifted = code << (bit & 31);
-      outw[bit >> 5] |= static_cast<uint32_t>(shifted);
-      if ((bit & 31) + bits > 32) outw[(bit >> 5) + 1] |= static_cast<uint32_t>(shifted >> 32);
-    }
-    for (int w = 0; w < bits; ++w) words[row * (static_cast<int64_t>(k) * bits / 32) + blk * bits + w] = outw[w];
-    if (blk < kg) {                                   // kg <= blocks: reuse the first kg threads of a row
-      const int g = blk;
-      const uint32_t v = tiled[(sb * kg + g) * unitw + TILE_PAIRS * 32 * wpl + affine_index(c)];
-      scales[row * kg + g] = static_cast<uint16_t>(v & 0xFFFFu);
-      biases[row * kg + g] = static_cast<uint16_t>(v >> 16);
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------------------------------------------------
 // group sums with the matmul kernel's own arithmetic: x against a tile of ones, one warp per (8 rows, group)
@@ -453,48 +370,6 @@ int tf_unit_words(int bits, int gs) { return format_ok(bits, gs) ? unit_words(bi
 int64_t tf_tiled_words(int n, int k, int bits, int gs) {
   if (!format_ok(bits, gs) || n < 1 || k < gs || k % gs) return TF_ERR_ARG;
   return static_cast<int64_t>((n + SB_COLS - 1) / SB_COLS) * (k / gs) * unit_words(bits, gs);
-}
-
-int tf_pack(const void* words, const void* scales, const void* biases, int n, int k, int bits, int gs, void* tiled,
-            void* stream) {
-  if (!format_ok(bits, gs)) return fail(TF_ERR_ARG, "tf_pack: %d bits / groups of %d is not an affine format", bits, gs);
-  if (n < 1 || k < gs || k % gs || (static_cast<int64_t>(k) * bits) % 32)
-    return fail(TF_ERR_ARG, "tf_pack: (%d, %d) does not split into whole groups and words", n, k);
-  if (!words || !scales || !biases || !tiled) return fail(TF_ERR_ARG, "tf_pack: null pointer");
-  const int64_t total = tf_tiled_words(n, k, bits, gs);
-  pack_kernel<<<grid_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint32_t*>(words), static_cast<const uint16_t*>(scales), static_cast<const uint16_t*>(biases), nullptr,
-      nullptr, nullptr, n, k, bits, gs, static_cast<uint32_t*>(tiled), total);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? TF_OK : cuda_fail(e, "tf_pack");
-}
-
-int tf_pack_pair(const void* words_a, const void* scales_a, const void* biases_a, const void* words_b, const void* scales_b,
-                 const void* biases_b, int n_each, int k, int bits, int gs, void* tiled, void* stream) {
-  if (!format_ok(bits, gs)) return fail(TF_ERR_ARG, "tf_pack_pair: %d bits / groups of %d is not an affine format", bits, gs);
-  if (n_each < 16 || n_each % 16 || k < gs || k % gs || (static_cast<int64_t>(k) * bits) % 32)
-    return fail(TF_ERR_ARG, "tf_pack_pair: (%d, %d) needs rows in whole 16-row tiles and whole groups and words", n_each, k);
-  if (!words_a || !scales_a || !biases_a || !words_b || !scales_b || !biases_b || !tiled)
-    return fail(TF_ERR_ARG, "tf_pack_pair: null pointer");
-  const int64_t total = tf_tiled_words(2 * n_each, k, bits, gs);
-  pack_kernel<<<grid_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint32_t*>(words_a), static_cast<const uint16_t*>(scales_a), static_cast<const uint16_t*>(biases_a),
-      static_cast<const uint32_t*>(words_b), static_cast<const uint16_t*>(scales_b), static_cast<const uint16_t*>(biases_b),
-      2 * n_each, k, bits, gs, static_cast<uint32_t*>(tiled), total);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? TF_OK : cuda_fail(e, "tf_pack_pair");
-}
-
-int tf_unpack(const void* tiled, int n, int k, int bits, int gs, void* words, void* scales, void* biases, void* stream) {
-  if (!format_ok(bits, gs)) return fail(TF_ERR_ARG, "tf_unpack: %d bits / groups of %d is not an affine format", bits, gs);
-  if (n < 1 || k < gs || k % gs || (static_cast<int64_t>(k) * bits) % 32)
-    return fail(TF_ERR_ARG, "tf_unpack: (%d, %d) does not split into whole groups and words", n, k);
-  if (!words || !scales || !biases || !tiled) return fail(TF_ERR_ARG, "tf_unpack: null pointer");
-  unpack_kernel<<<grid_for(static_cast<int64_t>(n) * (k / 32), 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint32_t*>(tiled), n, k, bits, gs, static_cast<uint32_t*>(words), static_cast<uint16_t*>(scales),
-      static_cast<uint16_t*>(biases));
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? TF_OK : cuda_fail(e, "tf_unpack");
 }
 
 int tf_group_sums(const void* x, int64_t ldx, int m, int k, int gs, float* xs, void* stream) {

@@ -38,6 +38,21 @@ def test_pack_round_trip_every_format(bits, gs):
     assert all(torch.equal(a, b) for a, b in zip(back, w))
 
 
+@pytest.mark.parametrize("bits", [2, 3, 4, 5, 6, 8])
+@pytest.mark.parametrize("gs", [32, 64, 128])
+def test_pack_runs_of_groups_and_pairs(bits, gs):
+    """37 groups: whole runs of groups and a ragged last one in every format; a gate/up pair is its rows interleaved."""
+
+    k = 37 * gs
+    a, b = (synthetic.raw_weight(144, k, bits, gs, seed) for seed in (bits, gs))
+    back = qmm.unpack(qmm.pack(*to_dev(*a), gs, bits=bits))
+    assert all(torch.equal(got.cpu(), want) for got, want in zip(back, a))
+    both = qmm.unpack(qmm.pack_pair(to_dev(*a), to_dev(*b), gs, bits))
+    for got, first, second in zip(both, a, b):
+        want = torch.stack([first.view(9, 16, -1), second.view(9, 16, -1)], 1).view(288, -1)
+        assert torch.equal(got.cpu(), want)
+
+
 @pytest.mark.parametrize("bits,gs", FORMATS)
 def test_exact_integer_case_is_bit_exact(bits, gs):
     """scale 0.25, bias -0.5, x in {-1, -.5, 0, .5, 1}: every product and sum is exact, so the output must be too."""
