@@ -172,11 +172,20 @@ int tf_moe_experts(const void* x, int64_t ldx, int slots, const void* tiled, int
                    int64_t ldo, int out_f32, int epi, float limit, void* stream);
 /* The same grouped projection in the prefill arithmetic (weights rounded once to bf16, one fp32 chain over K) on
  * tcgen05: the rows are first copied in member order into `sorted` ([pairs, k] bf16, caller scratch), then every item
- * (at most 128 pairs) runs as one tensor-memory tile per 128 output columns.  Plans for it use items of 128 pairs.
+ * (at most 128 pairs) runs as one tensor-memory tile per 256 output columns.  Plans for it use items of 128 pairs.
  * Replaces the pybind `prefill` of cuda/experts.cpp:69-82 (cuda/experts_prefill.cu:31-152). */
 int tf_moe_experts_prefill(const void* x, int64_t ldx, int slots, const void* tiled, int64_t expert_stride, int experts, int n,
                            int k, int gs, const int* items, const int* counts, const int* members, int pairs, int max_items,
                            void* sorted, void* out, int64_t ldo, int out_f32, int epi, float limit, void* stream);
+/* The two halves of tf_moe_experts_prefill, for a layer that keeps its activations in member order between its two
+ * projections.  tf_moe_gather: sorted[pos] = row members[pos] / slots of x (members[pos] with slots 0) for every planned
+ * pair.  tf_moe_experts_sorted: `sorted` holds the rows in member order, ldx elements apart; out row members[pos], or with
+ * members NULL row pos, which is the next projection's input as it stands. */
+int tf_moe_gather(const void* x, int64_t ldx, int slots, const int* items, const int* counts, const int* members, int pairs, int k,
+                  void* sorted, void* stream);
+int tf_moe_experts_sorted(const void* sorted, int64_t ldx, const void* tiled, int64_t expert_stride, int experts, int n, int k, int gs,
+                          const int* items, const int* counts, const int* members, int pairs, int max_items, void* out, int64_t ldo,
+                          int out_f32, int epi, float limit, void* stream);
 /* logits[r, e] = fp32 dot of bf16 rows x[r] and w[e].  Replaces the Triton `_router` of cuda/moe.py:23-55. */
 int tf_moe_router(const void* x, int64_t ldx, int rows, int d, const void* w, int ne, float* out, int64_t ldo, void* stream);
 /* The same logits in the prefill arithmetic: (16 rows x 16 experts) tensor-core tiles, K in order, fp32 accumulate.  A

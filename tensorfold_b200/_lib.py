@@ -44,6 +44,9 @@ SIGNATURES = {
                               ctypes.c_float, _vp)),
     "tf_moe_experts_prefill": (_i32, (_vp, _i64, _i32, _vp, _i64, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _i32, _vp, _vp, _i64,
                                       _i32, _i32, ctypes.c_float, _vp)),
+    "tf_moe_gather": (_i32, (_vp, _i64, _i32, _vp, _vp, _vp, _i32, _i32, _vp, _vp)),
+    "tf_moe_experts_sorted": (_i32, (_vp, _i64, _vp, _i64, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _i32, _vp, _i64, _i32, _i32,
+                                     ctypes.c_float, _vp)),
     "tf_selftest_lost_wait": (_i32, (_i32, _vp)),
     "tf_moe_router": (_i32, (_vp, _i64, _i32, _i32, _vp, _i32, _vp, _i64, _vp)),
     "tf_moe_router_tiles": (_i32, (_vp, _i64, _i32, _i32, _vp, _i32, _vp, _i64, _vp)),

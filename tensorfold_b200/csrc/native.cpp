@@ -32,7 +32,7 @@ namespace {
 #define TF_WRAPPED(X) X(tf_qmm) X(tf_qmm_set) X(tf_qmm_set_scratch_bytes) X(tf_qmm_prefill) X(tf_qmm_prefill_act) X(tf_qmm_act) \
   X(tf_add_rmsnorm) X(tf_swiglu)
 #define TF_THUNKS(X) X(tf_pack) X(tf_pack_pair) X(tf_unpack) X(tf_group_sums) X(tf_affine_rows) X(tf_moe_plan) X(tf_moe_experts) \
-  X(tf_moe_experts_prefill) X(tf_moe_router) X(tf_moe_router_tiles) X(tf_moe_topk) X(tf_moe_topk_local) X(tf_moe_combine)
+  X(tf_moe_experts_prefill) X(tf_moe_gather) X(tf_moe_experts_sorted) X(tf_moe_router) X(tf_moe_router_tiles) X(tf_moe_topk) X(tf_moe_topk_local) X(tf_moe_combine)
 
 #define TF_POINTER(name) decltype(&::name) p_##name = nullptr;
 TF_WRAPPED(TF_POINTER)

@@ -5,16 +5,27 @@
 // (tcgen05.mma, accumulator in tensor memory).  Any chunking of the rows gives the same bits; they are not the decode
 // kernel's bits (that one keeps the affine terms in fp32).
 //
-// Block tile = 128 output columns x 256 rows of x, "swap-AB": the dequantised weights are the MMA's A operand (M = 128),
-// the rows of x its B operand (N = 256), so every dequantised weight feeds 256 rows.  The kernel is persistent: a grid
-// no larger than the number of SMs, tiles dealt round-robin, and every producer simply runs on into the block's next
-// tile, so a tile's prologue (first bytes are about 2000 cycles away) and its drain overlap the neighbouring tiles'
-// MMAs.  Two rings decouple the latencies: packed units arrive from HBM by bulk copies into a ring of small slots; a
-// stage of the main ring holds the dequantised A tile and the x tile (a 2-D tensor-map copy with the 128-byte
-// swizzle) of 64 inputs behind ONE full barrier and ONE empty barrier.  Two accumulators in tensor memory alternate
-// between tiles.  Roles: warp 0 loads x, warp 1 owns tensor memory and issues the MMAs, warp 2 loads packed units,
-// warps 4-19 are two groups of eight conversion warps that take alternate stages (a stage's conversion is a long
-// dependent chain, so two stages are always in conversion), warps 20-23 drain the finished accumulator to global memory.
+// Two blocks (a cluster on one SM pair) share a tile of 256 output columns x up to 192 rows of x, "swap-AB": the
+// dequantised weights are the MMA's A operand (M = 256, 128 columns a block), the rows of x its B operand (N, half of them
+// in each block's shared memory), cta_group::2.  What bounds it is the tensor pipe, so everything else is kept below its
+// pace (2 N cycles a stage of 64 inputs):
+//   * A lives in TENSOR MEMORY: conversion warps hold their codes as m16n8k16 fragments already, one tcgen05.st.16x128b.x8 a
+//     warp and stage puts 16 columns x 64 inputs in place.  With A in shared memory (the first version: one block, 128 x 256
+//     tiles) a stage moved 105 KB through a port of 128 bytes a cycle, 823 cycles for 512 cycles of math; now it moves
+//     33 KB for 384 cycles of math;
+//   * the pair halves the bytes of x each SM brings in and reads;
+//   * two accumulators of 192 columns alternate between tiles (384 of the 512 tensor-memory columns; two 64-column stages of
+//     A take the rest, four beside accumulators of 128), so a tile's drain runs under the next tile's math;
+//   * N is chosen per call, or per expert, so that tiles fill the SM pairs in whole waves (see pf_rows).
+//
+// The kernel is persistent: tiles are dealt round-robin to at most one cluster an SM pair, and every producer runs on into
+// the next tile.  Rings: packed units (bulk copies, one super-block a block), x (tensor-map boxes), A stages.  Roles of a block: warp 0 loads x, warp 1 owns tensor memory and, in the first block of the pair,
+// issues the MMAs, warp 2 loads packed units, warps 4-19 are two groups of eight conversion warps that take alternate
+// stages, warps 20-27 drain the finished accumulator.  Barriers the MMA warp waits on live in the first block; the second
+// block's copies and conversion warps signal them across the pair.
+// Measured, one projection by CUDA events (in brackets one block a tile with A in shared memory): 2048 rows, 17408 x 5120
+// 246 us = 1484 TFLOP/s (335), 5120 x 17408 242 us (402), 1024 x 5120 21 us (53); 391 rows, 17408 x 5120 54 us (90); 64 rows,
+// 6144 x 5120 17 us (45).  cuBLAS does 8192^3 in bf16 at 1672 TFLOP/s here, 1424 over seconds: both are bound by power.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -33,40 +44,40 @@ int* device_error_word();          // tf_api.cu: the current device's error word
 
 namespace {
 
-constexpr int PF_COLS = 128;       // output columns of a block tile (MMA M)
-constexpr int PF_STAGE_K = 64;     // inputs a stage
-constexpr int PF_A_BYTES = PF_COLS * 128;
-constexpr int PF_W_BYTES = 5120;   // packed units of a stage: one g64 unit (4608 B) or two g32 units (5120 B)
-constexpr int PF_NW = 6;           // packed-unit slots in flight
-constexpr int PF_THREADS = 768;    // 24 warps: x loads, MMA, unit loads, (idle), 2 x 8 conversion, 4 drain
+constexpr int PF_COLS = 128;       // output columns of a block (half of the pair's MMA M)
+constexpr int PF_ROWS = 192;       // rows of x a tile may hold (MMA N)
+constexpr int PF_GROUP_ROWS = 128; // pairs a plan item may hold in the expert form
+constexpr int PF_STAGE_K = 128;    // inputs a stage: long enough that barrier traffic stays small beside the conversion
+constexpr int PF_XHALF = PF_ROWS / 2 * 128;        // a block's half of the rows, 64 inputs (128 bytes a row)
+constexpr int PF_X_BYTES = 2 * PF_XHALF;
+constexpr int PF_W_BYTES = 10240;  // packed units of a stage: two g64 units (9216 B) or four g32 units (10240 B)
+constexpr int PF_NX = 4;           // stages of x in flight
+constexpr int PF_NW = 10;          // packed-unit slots: 90 KB in flight an SM cover HBM's latency when experts stream once
+constexpr int PF_A_COLS = 64;      // tensor-memory columns of a stage of A
+constexpr int PF_TMEM_COLS = 512;  // two accumulators, then stages of A: two beside 192-column accumulators, four beside 128
+constexpr int PF_THREADS = 896;    // 28 warps: x loads, MMA, unit loads, (idle), 2 x 8 conversion, 8 drain
 constexpr int PF_CONV0 = 4;        // first conversion warp
-constexpr int PF_DRAIN0 = 20;      // first drain warp (a multiple of 4: tensor-memory lane groups go by warp % 4)
-constexpr int PF_BAR_BYTES = 512;
-
-// ROWS = rows of x of a block tile (MMA N): 256 for dense prompts, 128 for the grouped expert form
-template <int ROWS>
-struct PfGeo {
-  static constexpr int B_BYTES = ROWS * 128;
-  static constexpr int STAGE = PF_A_BYTES + B_BYTES;
-  static constexpr int NS = ROWS == 256 ? 4 : 6;           // stages in flight (even: the conversion groups alternate)
-  static constexpr int W_OFF = NS * STAGE, BAR_OFF = W_OFF + PF_NW * PF_W_BYTES;
-  static constexpr int SMEM = BAR_OFF + PF_BAR_BYTES + 1024 /* alignment slack */;
-  static_assert(STAGE % 1024 == 0, "tiles stay 1024-byte aligned for the 128-byte swizzle");
-  static_assert((2 * NS + 2 * PF_NW + 4) * 8 + 16 <= PF_BAR_BYTES, "barriers fit");
-  static_assert(NS % 2 == 0, "conversion groups alternate stages");
-  static_assert(SMEM <= 232448, "fits the opt-in shared memory of a block");
-};
+constexpr int PF_DRAIN0 = 20;      // first drain warp (multiples of 4: tensor-memory lane groups go by warp % 4)
+constexpr int PF_W_OFF = PF_NX * PF_X_BYTES, PF_BAR_OFF = PF_W_OFF + PF_NW * PF_W_BYTES;
+constexpr int PF_BARS = 2 * PF_NX + 2 * PF_NW + 4;
+constexpr int PF_SMEM = PF_BAR_OFF + PF_BARS * 8 + 16 + 1024 /* alignment slack */;
+static_assert(2 * PF_ROWS + 2 * PF_A_COLS <= PF_TMEM_COLS && 2 * 128 + 4 * PF_A_COLS <= PF_TMEM_COLS, "tensor memory");
+static_assert(PF_XHALF % 1024 == 0, "x tiles stay 1024-byte aligned for the 128-byte swizzle");
+static_assert(PF_NX == 4, "a stage of A (two or four of them) is released by the barrier of its x stage");
+static_assert(PF_SMEM <= 232448, "fits the opt-in shared memory of a block");
 
 struct PrefillParams {
   const uint32_t* w;
   int64_t sb_stride;
   int N, K, M;
+  int rows;                   // rows of a tile (a multiple of 16, at most PF_ROWS); the x map's boxes hold half of them
+  int acc_cols;               // columns of an accumulator: 128 or 192, at least `rows`
   void* out;
   int64_t ldo;
   int out_f32;
   int* err;
-  // grouped form (items != null): block (x, y) = plan item y = (expert, first, count <= ROWS); the tensor map covers the
-  // rows in member order, row first + r of it feeds pair members[first + r], which is the row of out that is written
+  // grouped form (items != null): a tile is plan item (expert, first, count <= rows) x 256 columns; row r of it is row
+  // first + r of x, which holds the rows in member order, and of out, or with members row members[first + r] of out
   const int* items;
   const int* counts;
   const int* members;
@@ -75,6 +86,15 @@ struct PrefillParams {
   int epi;                    // 0 store, 1 relu^2, 2 SwiGLU over gate/up rows interleaved in tiles of 16 (out: N / 2 columns)
   float limit;
 };
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// After a wait that gave up: copies in flight land before the shared memory is released.
+__device__ __forceinline__ void let_copies_land() {
+  for (int i = 0; i < 64; ++i) __nanosleep(20000);
+}
 
 __device__ __forceinline__ float pf_bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 __device__ __forceinline__ float pf_swiglu(float g, float u, float limit) {
@@ -94,107 +114,145 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_byte_addr) {
   return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
-// The whole warp runs these with warp-uniform operands (so the descriptors can live in uniform registers); the
-// instruction itself is predicated on `leader`, true in exactly one lane.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
-                                          uint32_t leader) {
+// One 16-input step of a stage: A [256 x 16] from tensor memory (128 lanes of each block), B [N x 16] from both blocks'
+// shared memory.  Issued by one thread.
+__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t leader) {
+// Arrives on the barrier at this address in both blocks of the pair once every MMA issued so far is done.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+
+// Bounded wait by a whole warp.  The polling loop stays out of line: the roles' loops share the
+// instruction caches, and a role that misses there waits hundreds of cycles for a handful of instructions.
+__device__ __noinline__ bool poll(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < WAIT_POLLS; ++i) {
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity), "r"(20000u)
+                 : "memory");
+    if (done) return true;
+    if ((i & 255u) == 255u && *abort_flag) return false;
+  }
+  return false;
+}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
+  if (__all_sync(0xFFFFFFFFu, mbar32_try_wait(bar, parity))) return true;
+  return __all_sync(0xFFFFFFFFu, poll(bar, parity, abort_flag));
+}
+
+// Sixteen columns of output x 64 inputs: register 4 s + j of a lane is its A-fragment register j of 16-input step s.
+__device__ __forceinline__ void tmem_store_a(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
-      "{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_addr(bar)),
-      "r"(leader)
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
+// True in one lane of the warp.
+__device__ __forceinline__ bool elect() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
+}
+
+// The address of a barrier in the first block of the pair.
+__device__ __forceinline__ uint32_t in_first(const void* p) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_addr(p)));
+  return remote;
+}
+__device__ __forceinline__ void arrive_first(uint32_t remote) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
+// Tensor-map copies into this block's shared memory that complete on a barrier of the first block.
+__device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+               "l"(map), "r"(bar), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[2][8]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, "
-      "%18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=f"(v[0][0]), "=f"(v[0][1]), "=f"(v[0][2]), "=f"(v[0][3]), "=f"(v[0][4]), "=f"(v[0][5]), "=f"(v[0][6]), "=f"(v[0][7]),
+        "=f"(v[1][0]), "=f"(v[1][1]), "=f"(v[1][2]), "=f"(v[1][3]), "=f"(v[1][4]), "=f"(v[1][5]), "=f"(v[1][6]), "=f"(v[1][7])
       : "r"(taddr)
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-template <int GS, int ROWS>
+// Eight lanes each hold eight rows of one column; afterwards each holds eight columns of one row, as bf16: lane l of the
+// group gets row l.  Rows are rounded and paired first, so three exchanges of two words do it.
+__device__ __forceinline__ uint4 transpose8(const float (&v)[8], int lane) {
+  uint32_t p[4];                                             // rows 2 i, 2 i + 1 of this lane's column
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    p[i] = *reinterpret_cast<const uint32_t*>(&t);
+  }
+  // neighbouring columns: an even lane keeps rows 2 i of both, an odd lane rows 2 i + 1
+  const bool odd = lane & 1;
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {
+    const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, __byte_perm(p[i], p[i + 1], odd ? 0x5410 : 0x7632), 1);
+    p[i] = odd ? __byte_perm(got, p[i], 0x7610) : __byte_perm(p[i], got, 0x5410);
+    p[i + 1] = odd ? __byte_perm(got, p[i + 1], 0x7632) : __byte_perm(p[i + 1], got, 0x7610);
+  }
+  // then a 4 x 4 transpose of (column pair, row pair) words over the other two lane bits
+#pragma unroll
+  for (int bit = 1; bit <= 2; bit <<= 1) {
+    const bool upper = lane & (2 * bit);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i & bit) continue;
+      const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? p[i] : p[i | bit], 2 * bit);
+      if (upper) p[i] = got;
+      else p[i | bit] = got;
+    }
+  }
+  return make_uint4(p[0], p[1], p[2], p[3]);
+}
+
+template <int GS>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_constant__ CUtensorMap tmx, const PrefillParams p) {
-  using Geo = PfGeo<ROWS>;
-  constexpr int PF_ROWS = ROWS, PF_B_BYTES = Geo::B_BYTES, NS = Geo::NS;
-  constexpr uint32_t PF_TMEM_COLS = 2 * ROWS;                // two accumulators: one fills while the other drains
   constexpr int S = GS / 16;                                 // k16 steps a group
-  constexpr int UNITS = PF_STAGE_K / GS;                     // units a stage (1 for g64, 2 for g32)
+  constexpr int UNITS = PF_STAGE_K / GS;                     // units a stage (2 for g64, 4 for g32)
   constexpr int WPL = words_per_lane(4, GS);
   constexpr int UNITW = unit_words(4, GS);
   static_assert(UNITS * UNITW * 4 <= PF_W_BYTES, "slot holds a stage's packed units");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Geo::BAR_OFF);
-  uint64_t* full = bars;                            // stage ready: 8 conversion warps arrived and the x tile landed
-  uint64_t* empty = full + NS;                      // the MMAs that read the stage are done
-  uint64_t* w_full = empty + NS;                    // packed units landed (bulk copy)
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + PF_BAR_OFF);     // first block: the pair's rows of x have landed and its 16
+                                                    // conversion warps have stored their A
+  uint64_t* empty = full + PF_NX;                   // the MMAs that read the stage (x and A) are done
+  uint64_t* w_full = empty + PF_NX;                 // packed units landed (bulk copy)
   uint64_t* w_empty = w_full + PF_NW;               // the 8 conversion warps of the stage's group have read the slot
   uint64_t* acc_full = w_empty + PF_NW;             // [2] every MMA of a tile is done
-  uint64_t* acc_empty = acc_full + 2;               // [2] the 4 drain warps have read the accumulator
+  uint64_t* acc_empty = acc_full + 2;               // [2] first block: the 16 drain warps of the pair have read the accumulator
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  const int half = blockIdx.x & 1, pair_id = blockIdx.x >> 1, pairs_in_grid = gridDim.x >> 1;     // (clusters are blocks 2 i, 2 i + 1)
   const int nstages = (p.K + PF_STAGE_K - 1) / PF_STAGE_K;
   const int total_units = p.K / GS;
-  const int nsb = (p.N + PF_COLS - 1) / PF_COLS;
+  const int nsb = (p.N + PF_COLS - 1) / PF_COLS, ncp = (nsb + 1) / 2;
   const bool grouped = p.items != nullptr;
-  // Tiles = column blocks x row tiles (plan items in the grouped form), column block fastest, dealt round-robin to the
-  // blocks of a grid no larger than the number of SMs.  Every role walks the same (tile, stage) sequence, so a running
-  // stage count g names the ring slot (g % NS) and its phase without any exchange between the roles.
-  const int row_tiles = grouped ? p.counts[0] : (p.M + PF_ROWS - 1) / PF_ROWS;
-  const int tiles = nsb * row_tiles;
-  const int first_tile = blockIdx.x;
-  if (first_tile >= tiles) return;                           // before any barrier or tensor-memory use
-  const int my_tiles = (tiles - first_tile + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
-  const int total = my_tiles * nstages;                      // stages this block runs
+  const int a_stages = p.acc_cols > 128 ? 2 : 4;
+  const uint32_t a_col0 = 2 * p.acc_cols;
 
-  struct Tile {
-    int sb, m0, rows_here, first;
-    const uint32_t* wroot;
-  };
-  auto tile_at = [&](int it) {
-    const int t = first_tile + it * static_cast<int>(gridDim.x);
-    Tile ti;
-    ti.sb = t % nsb;
-    const int y = t / nsb;
-    ti.wroot = p.w;
-    if (grouped) {
-      const int* item = p.items + 3 * y;
-      // an item that names an expert outside the table runs against expert 0 with no rows (nothing is stored) and
-      // is reported: every role still walks the same tile sequence, and nothing is read past the table
-      const bool known = item[0] >= 0 && item[0] < p.experts;
-      if (!known && threadIdx.x == 0) atomicCAS(p.err, 0, ERR_BAD_ITEM);
-      ti.wroot += static_cast<int64_t>(known ? item[0] : 0) * p.expert_stride;
-      ti.first = item[1];
-      ti.rows_here = known ? min(PF_ROWS, item[2]) : 0;
-      ti.m0 = item[1];                                       // row of the member-ordered input
-    } else {
-      ti.first = 0;
-      ti.m0 = y * PF_ROWS;
-      ti.rows_here = min(PF_ROWS, p.M - ti.m0);
-    }
-    return ti;
-  };
-
-  auto a_tile = [&](int s) { return smem + s * Geo::STAGE; };
-  auto b_tile = [&](int s) { return smem + s * Geo::STAGE + PF_A_BYTES; };
-  auto w_slot = [&](int s) { return smem + Geo::W_OFF + s * PF_W_BYTES; };
   auto give_up = [&](int code) {
     if (lane == 0) {
       *abort_flag = code;
@@ -203,280 +261,317 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
   };
 
   if (tid == 0) {
-    for (int i = 0; i < NS; ++i) mbar_init(full + i, 9), mbar_init(empty + i, 1);
+    for (int i = 0; i < PF_NX; ++i) mbar_init(full + i, 17), mbar_init(empty + i, 1);
     for (int i = 0; i < PF_NW; ++i) mbar_init(w_full + i, 1), mbar_init(w_empty + i, 8);
-    for (int i = 0; i < 2; ++i) mbar_init(acc_full + i, 1), mbar_init(acc_empty + i, 4);
+    for (int i = 0; i < 2; ++i) mbar_init(acc_full + i, 1), mbar_init(acc_empty + i, 16);
     *abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(PF_TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)), "r"(PF_TMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();                                            // the pair's barriers exist before either block signals the other
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();
+
+  // Tiles = pairs of column blocks x row tiles (plan items in the grouped form), columns fastest, dealt round-robin to the
+  // clusters.  Every role of both blocks walks the same (tile, stage) sequence, so a running stage count g names the ring
+  // slots and their phases without any exchange between the roles.
+  if (grouped) pdl_wait();                                   // the plan may be the previous kernel's output
+  const int row_tiles = grouped ? p.counts[0] : (p.M + p.rows - 1) / p.rows;
+  const int tiles = ncp * row_tiles;
+  const int my_tiles = pair_id < tiles ? (tiles - pair_id + pairs_in_grid - 1) / pairs_in_grid : 0;
+  const int total = my_tiles * nstages;                      // stages this block runs
+
+  struct Tile {
+    int sb;                                                  // this block's super-block (past the last one: nothing is stored)
+    int m0, rows_here, n;                                    // first row (of members in the grouped form), rows, MMA N
+    const uint32_t* w;                                       // this block's units
+  };
+  auto tile_at = [&](int it) {
+    const int t = pair_id + it * pairs_in_grid;
+    const int y = t / ncp;
+    Tile ti;
+    ti.sb = 2 * (t - y * ncp) + half;
+    ti.w = p.w + static_cast<int64_t>(min(ti.sb, nsb - 1)) * p.sb_stride;
+    if (grouped) {
+      const int* item = p.items + 3 * y;
+      // an item that names an expert outside the table runs against expert 0 with no rows (nothing is stored) and is
+      // reported: every role still walks the same tile sequence, and nothing is read past the table
+      const int expert = __ldg(item);
+      const bool known = expert >= 0 && expert < p.experts;
+      if (!known && threadIdx.x == 0) atomicCAS(p.err, 0, ERR_BAD_ITEM);
+      ti.w += static_cast<int64_t>(known ? expert : 0) * p.expert_stride;
+      ti.m0 = __ldg(item + 1);
+      ti.rows_here = known ? min(p.rows, __ldg(item + 2)) : 0;
+    } else {
+      ti.m0 = y * p.rows;
+      ti.rows_here = min(p.rows, p.M - ti.m0);
+    }
+    ti.n = max(16, (ti.rows_here + 15) & ~15);
+    return ti;
+  };
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ x tiles (L2 -> shared, tensor-map copies)
+    // ------------------------------------------------------------------ x tiles (L2 -> shared): this block's half of the rows
+    if (!grouped) pdl_wait();                                // x may be the previous kernel's output
     bool ok = true;
-    int g = 0;
+    int slot = 0;
+    uint32_t phase = 1;                                      // parity of the `empty` phase that frees the slot (first round: passes)
+    const uint32_t bytes = p.rows * 128;                     // both blocks' copies of 64 inputs
+    const uint32_t full0 = in_first(full), full32 = smem_addr(full), empty32 = smem_addr(empty), smem32 = smem_addr(smem);
     for (int it = 0; it < my_tiles && ok; ++it) {
       const Tile ti = tile_at(it);
-      for (int ls = 0; ls < nstages && ok; ++ls, ++g) {
-        const int s = g % NS;
-        if (g >= NS) {
-          ok = mbar_wait(empty + s, (g / NS - 1) & 1, abort_flag);
-          if (!ok) {
-            give_up(ERR_WAIT_EMPTY);
-            break;
-          }
-        }
-        if (lane == 0) {
-          mbar_expect_tx(full + s, PF_B_BYTES);
-          tma_load_2d(b_tile(s), &tmx, ls * PF_STAGE_K, ti.m0, full + s);
+      const int y = ti.m0 + half * (ti.n / 2);               // (a box may reach past the share: those rows are not multiplied)
+#pragma unroll 1
+      for (int ls = 0; ls < nstages; ++ls) {
+        ok = warp_wait(empty32 + 8 * slot, phase, abort_flag);
+        if (!ok) break;
+        const uint32_t bar = full0 + 8 * slot, dst = smem32 + slot * PF_X_BYTES;
+        const int k0 = ls * PF_STAGE_K;
+        const bool both = p.K - k0 > 64;
+        if (elect()) {
+          if (half == 0) mbar32_expect_tx(full32 + 8 * slot, both ? 2 * bytes : bytes);
+          pair_load_2d(dst, &tmx, k0, y, bar);
+          if (both) pair_load_2d(dst + PF_XHALF, &tmx, k0 + 64, y, bar);
         }
         __syncwarp();
+        if (++slot == PF_NX) slot = 0, phase ^= 1u;
       }
     }
+    if (!ok) give_up(ERR_WAIT_EMPTY);
+    if (!ok) let_copies_land();
   } else if (warp == 2) {
     // ------------------------------------------------------------------ packed units (HBM -> shared, bulk copies)
     bool ok = true;
-    int g = 0;
+    int slot = 0;
+    uint32_t phase = 1;
+    const uint32_t w_full32 = smem_addr(w_full), w_empty32 = smem_addr(w_empty), smem32 = smem_addr(smem + PF_W_OFF);
     for (int it = 0; it < my_tiles && ok; ++it) {
-      const Tile ti = tile_at(it);
-      const uint32_t* wsb = ti.wroot + static_cast<int64_t>(ti.sb) * p.sb_stride;
-      for (int ls = 0; ls < nstages && ok; ++ls, ++g) {
-        const int s = g % PF_NW;
-        if (g >= PF_NW) {
-          ok = mbar_wait(w_empty + s, (g / PF_NW - 1) & 1, abort_flag);
-          if (!ok) {
-            give_up(ERR_WAIT_EMPTY);
-            break;
-          }
-        }
-        if (lane == 0) {
-          const int units_here = min(UNITS, total_units - ls * UNITS);
-          mbar_expect_tx(w_full + s, units_here * UNITW * 4);
-          bulk_load(w_slot(s), wsb + static_cast<int64_t>(ls) * UNITS * UNITW, units_here * UNITW * 4, w_full + s);
+      const uint32_t* w = tile_at(it).w;
+#pragma unroll 1
+      for (int ls = 0; ls < nstages; ++ls, w += UNITS * UNITW) {
+        ok = warp_wait(w_empty32 + 8 * slot, phase, abort_flag);
+        if (!ok) break;
+        const uint32_t bytes = min(UNITS, total_units - ls * UNITS) * UNITW * 4;
+        if (elect()) {
+          mbar32_expect_tx(w_full32 + 8 * slot, bytes);
+          bulk_load32(smem32 + slot * PF_W_BYTES, w, bytes, w_full32 + 8 * slot);
         }
         __syncwarp();
+        if (++slot == PF_NW) slot = 0, phase ^= 1u;
       }
     }
+    if (!ok) give_up(ERR_WAIT_EMPTY);
+    if (!ok) let_copies_land();
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issue (one thread)
-    // The tensor pipe's queue is short and every instruction of this warp between two MMA issues is dead time for
-    // it, so the loop is unrolled over the ring (descriptors by constant offsets, no index arithmetic) and the next
-    // stage's full barrier is tested between this stage's MMAs, while earlier ones are still executing.
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((PF_ROWS >> 3) << 17) | ((PF_COLS >> 4) << 24);
-    constexpr uint64_t SLOT_STEP = Geo::STAGE >> 4;            // a ring slot further, in descriptor address units
-    const uint32_t leader = lane == 0 ? 1u : 0u;
-    const uint64_t ad0 = umma_desc(smem_addr(a_tile(0))), bd0 = umma_desc(smem_addr(b_tile(0)));
-    bool ok = mbar_wait(full, 0, abort_flag);
-    if (!ok) give_up(ERR_WAIT_FULL);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t phase = 0;                                          // parity of the full barriers of this pass over the ring
-    int ls = 0, it = 0;                                          // stage inside the tile, tile count of this block
-    for (int base = 0; base < total && ok; base += NS, phase ^= 1u) {
+    // ------------------------------------------------------------------ MMA issue (one thread of the first block)
+    if (half == 0) {
+      // The tensor pipe's queue is short, so this warp must stay ahead of it: one barrier a stage, eight MMAs a barrier,
+      // and addresses that are the same in every lane (elect.sync lets the compiler keep them in uniform registers:
+      // 32 cycles an MMA of 64 rows against 78 for a loop behind `lane == 0`).
+      const uint32_t full32 = smem_addr(full), empty32 = smem_addr(empty), acc_full32 = smem_addr(acc_full);
+      const uint64_t bd0 = umma_desc(smem_addr(smem));
+      const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+      const int whole = p.K / PF_STAGE_K;                      // stages of 128 inputs; K may end with half of one
+      bool ok = true;
+      int slot = 0;
+      uint32_t phase = 0, a_slot = 0;
+      for (int it = 0; it < my_tiles && ok; ++it) {
+        const uint32_t n8 = __shfl_sync(0xFFFFFFFFu, static_cast<uint32_t>(tile_at(it).n >> 3), 0);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (n8 << 17) | ((256u >> 4) << 24);
+        const uint32_t acc = tmem + static_cast<uint32_t>((it & 1) * p.acc_cols);
+        // the accumulator's last tile must have been drained
+        if (it >= 2) ok = warp_wait(smem_addr(acc_empty + (it & 1)), ((it >> 1) - 1) & 1, abort_flag);
+#pragma unroll 1
+        for (int ls = 0; ls < nstages && ok; ++ls) {
+          ok = warp_wait(full32 + 8 * slot, phase, abort_flag);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a = tmem + a_col0 + a_slot * PF_A_COLS;
+          const uint64_t bd = bd0 + slot * (PF_X_BYTES >> 4);
+          if (elect()) {
+            umma_pair(acc, a, bd, idesc, ls != 0 ? 1u : 0u);   // 16 inputs: 8 columns of A, 32 bytes inside the swizzle atom
 #pragma unroll
-      for (int st = 0; st < NS; ++st) {
-        const int g = base + st;
-        if (g >= total || !ok) break;
-        if (ls == 0 && it >= 2) {                                // the accumulator's last tile must have been drained
-          ok = mbar_wait(acc_empty + (it & 1), ((it >> 1) - 1) & 1, abort_flag);
-          if (!ok) {
-            give_up(ERR_WAIT_EMPTY);
-            break;
+            for (int q = 1; q < 4; ++q) umma_pair(acc, a + 8 * q, bd + 2 * q, idesc, 1u);
+            if (ls < whole || p.K % PF_STAGE_K > 64) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) umma_pair(acc, a + 32 + 8 * q, bd + (PF_XHALF >> 4) + 2 * q, idesc, 1u);
+            }
+            umma_commit_pair(empty32 + 8 * slot);
+            if (ls == nstages - 1) umma_commit_pair(acc_full32 + 8 * (it & 1));
           }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        const uint32_t acc = tmem_base + static_cast<uint32_t>(it & 1) * PF_ROWS;
-        const uint64_t ad = ad0 + st * SLOT_STEP, bd = bd0 + st * SLOT_STEP;
-        const int nx = (st + 1) % NS;
-        const uint32_t nx_phase = st + 1 == NS ? phase ^ 1u : phase;
-        const bool more = g + 1 < total;
-        bool next_ready = false;
-        umma_bf16(acc, ad, bd, IDESC, ls > 0 ? 1u : 0u, leader);
-        umma_bf16(acc, ad + 2, bd + 2, IDESC, 1u, leader);       // + 32 bytes a k16 step inside the swizzle atom
-        umma_bf16(acc, ad + 4, bd + 4, IDESC, 1u, leader);
-        if (more) {
-          next_ready = mbar_test(full + nx, nx_phase);
-          if (next_ready) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        umma_bf16(acc, ad + 6, bd + 6, IDESC, 1u, leader);
-        umma_commit(empty + st, leader);
-        if (ls == nstages - 1) {
-          umma_commit(acc_full + (it & 1), leader);
-          ls = 0, ++it;
-        } else {
-          ++ls;
-        }
-        if (more && !next_ready) {
-          ok = mbar_wait(full + nx, nx_phase, abort_flag);
-          if (!ok) give_up(ERR_WAIT_FULL);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          __syncwarp();
+          a_slot = (a_slot + 1) & (a_stages - 1);
+          if (++slot == PF_NX) slot = 0, phase ^= 1u;
         }
       }
+      if (!ok) give_up(ERR_WAIT_FULL);
     }
   } else if (warp >= PF_CONV0 && warp < PF_DRAIN0) {
-    // ------------------------------------------------------------------ conversion: packed codes -> swizzled bf16 A tile
-    // A warp owns 16 output columns (tile pair tp, half h) of every stage its group takes.  Per 16-input step a thread
-    // holds the four m8n8 fragments (two column octets x two input octets) of its lane's codes, so one stmatrix.x4
-    // writes four 8 x 16-byte row segments of the swizzled tile; lane l supplies the address of row l % 8 of fragment l / 8.
+    // ------------------------------------------------------------------ conversion: packed codes -> bf16 A stage in tensor memory
+    // A warp owns 16 output columns (tile pair tp, half h) of every stage its group takes; its lanes hold the codes as
+    // A fragments, which is how tcgen05.st.16x128b lays them down (lane = output column, 32-bit column = two inputs).
     const int cw = warp - PF_CONV0, group = cw >> 3, dw = cw & 7, tp = dw & 3, h = dw >> 2, g8 = lane >> 2;
     const __nv_bfloat162 k128 = __floats2bfloat162_rn(128.f, 128.f);
-    uint32_t row_off[4];                                        // this lane's row segment of each 16-input step of a stage
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      row_off[q] = (32 * tp + 16 * h + 8 * ((lane >> 3) & 1) + (lane & 7)) * 128 + (((2 * q + (lane >> 4)) ^ (lane & 7)) << 4);
+    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(32 * tp + 16 * h) << 16) + a_col0;
+    const uint32_t full0 = in_first(full);
+    const uint32_t w_off = smem_addr(smem + PF_W_OFF) + ((tp * 32 + lane) * WPL + h * S) * 4;
+    const uint32_t sb_off = smem_addr(smem + PF_W_OFF) + (TILE_PAIRS * 32 * WPL + tp * 32 + g8 * 4 + h * 2) * 4;
     bool ok = true;
-    for (int i = group; i < total && ok; i += 2) {             // i = the block's running stage count
-      const int sw = i % PF_NW, st = i % NS, ls = i % nstages;
-      ok = mbar_wait(w_full + sw, (i / PF_NW) & 1, abort_flag);
-      if (ok && i >= NS) ok = mbar_wait(empty + st, (i / NS - 1) & 1, abort_flag);
+    int sw = group, ls = group % nstages;
+    uint32_t pw = 0;
+    for (int i = group; i < total; i += 2) {                   // i = the block's running stage count
+      ok = warp_wait(smem_addr(w_full + sw), pw, abort_flag);
       if (!ok) {
         give_up(ERR_WAIT_FULL);
         break;
       }
-      const uint32_t* wst = reinterpret_cast<const uint32_t*>(w_slot(sw));
-      const uint32_t at = smem_addr(a_tile(st));
-      const int units_here = min(UNITS, total_units - ls * UNITS);
+      const int units_here = total_units - ls * UNITS;         // (of UNITS: K may end inside the stage)
+      uint32_t frag[2][16];
 #pragma unroll
       for (int u = 0; u < UNITS; ++u) {
-        uint32_t wd[S] = {};
+        const uint32_t at = sw * PF_W_BYTES + u * UNITW * 4;
+        uint32_t wd[S];
+        if constexpr (S == 4) {
+          const uint4 v = lds128(w_off + at);
+          wd[0] = v.x, wd[1] = v.y, wd[2] = v.z, wd[3] = v.w;
+        } else {
+          const uint2 v = lds64(w_off + at);
+          wd[0] = v.x, wd[1] = v.y;
+        }
+        uint2 sbw = lds64(sb_off + at);                        // columns g8 and g8 + 8 of the half
+        // past the end of K x is zero (the tensor map fills it) and the weights must be finite: scales and biases of
+        // zero give zero weights
+        if (u > 0 && u >= units_here) sbw = make_uint2(0u, 0u);
         __nv_bfloat162 sc[2], bi[2];
-        sc[0] = sc[1] = bi[0] = bi[1] = __floats2bfloat162_rn(0.f, 0.f);
-        // past the end of K (it ends inside this stage) x is zero (the tensor map fills it) and the weights must be
-        // finite: codes, scales and biases of zero give zero weights
-        if (u < units_here) {
-          const uint32_t* unit = wst + u * UNITW;
-          if constexpr (S == 4) {
-            const uint4 v = *reinterpret_cast<const uint4*>(unit + (tp * 32 + lane) * WPL + h * S);
-            wd[0] = v.x, wd[1] = v.y, wd[2] = v.z, wd[3] = v.w;
-          } else {
-            const uint2 v = *reinterpret_cast<const uint2*>(unit + (tp * 32 + lane) * WPL + h * S);
-            wd[0] = v.x, wd[1] = v.y;
-          }
-          const uint2 sbw = *reinterpret_cast<const uint2*>(unit + TILE_PAIRS * 32 * WPL + tp * 32 + g8 * 4 + h * 2);
-          const uint32_t sbv[2] = {sbw.x, sbw.y};                  // columns c0 and c0 + 8
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const uint32_t s2 = __byte_perm(sbv[r], 0u, 0x1010), b2 = __byte_perm(sbv[r], 0u, 0x3232);
-            sc[r] = *reinterpret_cast<const __nv_bfloat162*>(&s2);
-            bi[r] = *reinterpret_cast<const __nv_bfloat162*>(&b2);
-          }
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t v = r == 0 ? sbw.x : sbw.y, s2 = __byte_perm(v, 0u, 0x1010), b2 = __byte_perm(v, 0u, 0x3232);
+          sc[r] = *reinterpret_cast<const __nv_bfloat162*>(&s2);
+          bi[r] = *reinterpret_cast<const __nv_bfloat162*>(&b2);
         }
 #pragma unroll
-        for (int sidx = 0; sidx < S; ++sidx) {
-          uint32_t frag[4];
+        for (int sidx = 0; sidx < S; ++sidx)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            uint32_t v = ((wd[sidx] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
+            uint32_t v = lop3_and_or(wd[sidx] >> (4 * j), 0x000F000Fu, 0x43004300u);
             const __nv_bfloat162 q2 = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), k128);       // exact code
             const __nv_bfloat162 w2 = __hfma2(q2, sc[j & 1], bi[j & 1]);                            // one rounding
-            frag[j] = *reinterpret_cast<const uint32_t*>(&w2);
+            frag[u * S / 4][(u * S % 4 + sidx) * 4 + j] = *reinterpret_cast<const uint32_t*>(&w2);
           }
-          asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(at + row_off[u * S + sidx]),
-                       "r"(frag[0]), "r"(frag[1]), "r"(frag[2]), "r"(frag[3])
-                       : "memory");
-        }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the tensor core's reads
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(full + st);
-        mbar_arrive(w_empty + sw);                               // the slot's words are in registers or already used
+      if (elect()) mbar_arrive(w_empty + sw);                // the slot's words are in registers
+      if (i >= a_stages) {                                     // the MMAs that read the A stage's last contents are done
+        const int before = i - a_stages;
+        ok = warp_wait(smem_addr(empty + before % PF_NX), (before / PF_NX) & 1, abort_flag);
+        if (!ok) {
+          give_up(ERR_WAIT_EMPTY);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
+      const uint32_t a = a_lane + (i & (a_stages - 1)) * PF_A_COLS;
+      tmem_store_a(a, frag[0]);
+      if (units_here * GS > 64) tmem_store_a(a + 32, frag[1]);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (elect()) arrive_first(full0 + 8 * (i % PF_NX));
+      sw += 2;
+      if (sw >= PF_NW) sw -= PF_NW, pw ^= 1u;
+      ls += 2;
+      while (ls >= nstages) ls -= nstages;
     }
   } else if (warp >= PF_DRAIN0) {
     // ------------------------------------------------------------------ drain: tensor memory -> global, a tile behind
-    const int lg = warp & 3;                                   // this warp may touch TMEM lanes [32 lg, 32 lg + 32)
+    if (!grouped) pdl_wait();                                  // nothing is written before the previous kernel is done
+    const int lg = warp & 3, part = (warp - PF_DRAIN0) >> 2;   // this warp may touch TMEM lanes [32 lg, 32 lg + 32)
+    const uint32_t acc_empty0 = in_first(acc_empty);
     for (int it = 0; it < my_tiles; ++it) {
       const Tile ti = tile_at(it);
-      const int ab = it & 1, rows_here = ti.rows_here, first = ti.first, m0 = ti.m0, sb = ti.sb;
-      const bool done = mbar_wait(acc_full + ab, (it >> 1) & 1, abort_flag);
+      const int ab = it & 1, rows_here = ti.rows_here, m0 = ti.m0, sb = ti.sb;
+      const bool done = warp_wait(smem_addr(acc_full + ab), (it >> 1) & 1, abort_flag);
       if (!done) {
         give_up(ERR_WAIT_FULL);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (*abort_flag != 0) break;
-      // A lane holds one output column for 32 rows of x.  Each group of eight lanes transposes its 8 x 8 blocks in
-      // registers (three butterfly steps), so a lane then holds eight neighbouring columns of one row and writes them
-      // as 16 bytes: a store instruction costs about the same whatever its width, and narrow ones made the drain the
-      // slowest part of a tile.
+      // Sixteen rows of x a pass, passes in turn between the two warps of a lane group.  A lane holds its output column for
+      // them; each group of eight lanes transposes 8 x 8 blocks in registers, so that a lane writes eight neighbouring
+      // columns of one row as 16 bytes.
       const bool swiglu = p.epi == 2;
-      const int col = swiglu ? sb * (PF_COLS / 2) + lg * 16 + lane : sb * PF_COLS + lg * 32 + lane;
+      const int col = swiglu ? sb * (PF_COLS / 2) + lg * 16 + (lane & 15) : sb * PF_COLS + lg * 32 + lane;
       const int ncols = swiglu ? p.N / 2 : p.N;
-      const bool live = col < ncols && (!swiglu || lane < 16);
+      const bool live = sb < nsb && col < ncols;
       const bool wide = !p.out_f32 && (ncols & 7) == 0 && (p.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
-      const int l8 = lane & 7;
-#pragma unroll 1
-      for (int col0 = 0; col0 < rows_here; col0 += 32) {         // 32 rows of x a pass
-        uint32_t r[32];
-        tmem_load32(tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + static_cast<uint32_t>(ab * PF_ROWS + col0), r);
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          v[j] = __uint_as_float(r[j]);
-          if (swiglu) {                                          // lanes 0-15 hold gate columns, 16-31 the up columns
-            const float up = __shfl_down_sync(0xFFFFFFFFu, v[j], 16);
-            v[j] = pf_swiglu(v[j], up, p.limit);
-          } else if (p.epi == 1) {
-            v[j] = fmaxf(pf_bf16r(v[j]), 0.f);
-            v[j] = v[j] * v[j];
-          }
-        }
+      const uint32_t acc = tmem_base + (static_cast<uint32_t>(lg * 32) << 16) + static_cast<uint32_t>(ab * p.acc_cols);
+      // v[j] = output column `col` of row rr + j
+      auto store8 = [&](const float (&v)[8], int rr) {
         if (wide) {
-#pragma unroll
-          for (int blk = 0; blk < 4; ++blk) {                    // rows 8 blk .. 8 blk + 7 of the pass
-            float* a = v + 8 * blk;
-#pragma unroll
-            for (int mask = 4; mask >= 1; mask >>= 1) {
-              const bool upper = (l8 & mask) != 0;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                if (i & mask) continue;
-                const float got = __shfl_xor_sync(0xFFFFFFFFu, upper ? a[i] : a[i | mask], mask);
-                if (upper) a[i] = got;
-                else a[i | mask] = got;
-              }
-            }
-            const int rr = col0 + 8 * blk + l8;                  // a[c] = column (col - l8 + c) of row rr
-            if (live && rr < rows_here) {
-              const int64_t m = grouped ? p.members[first + rr] : m0 + rr;
-              uint4 o;
-              __nv_bfloat162 t0 = __floats2bfloat162_rn(a[0], a[1]), t1 = __floats2bfloat162_rn(a[2], a[3]);
-              __nv_bfloat162 t2 = __floats2bfloat162_rn(a[4], a[5]), t3 = __floats2bfloat162_rn(a[6], a[7]);
-              o.x = *reinterpret_cast<uint32_t*>(&t0), o.y = *reinterpret_cast<uint32_t*>(&t1);
-              o.z = *reinterpret_cast<uint32_t*>(&t2), o.w = *reinterpret_cast<uint32_t*>(&t3);
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + m * p.ldo + (col - l8)) = o;
-            }
+          const uint4 o = transpose8(v, lane);                 // columns col - l8 .. col - l8 + 7 of row rr + l8
+          const int r = rr + (lane & 7);
+          if (live && r < rows_here) {
+            const int64_t m = p.members != nullptr ? p.members[m0 + r] : m0 + r;
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + m * p.ldo + (col - (lane & 7))) = o;
           }
         } else if (live) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int rr = col0 + j;
-            if (rr < rows_here) {
-              const int64_t m = grouped ? p.members[first + rr] : m0 + rr;
+          for (int j = 0; j < 8; ++j) {
+            if (rr + j < rows_here) {
+              const int64_t m = p.members != nullptr ? p.members[m0 + rr + j] : m0 + rr + j;
               if (p.out_f32) reinterpret_cast<float*>(p.out)[m * p.ldo + col] = v[j];
               else reinterpret_cast<__nv_bfloat16*>(p.out)[m * p.ldo + col] = __float2bfloat16_rn(v[j]);
             }
           }
         }
+      };
+#pragma unroll 1
+      for (int r0 = 16 * part; r0 < rows_here; r0 += 32) {
+        float v[2][8];
+        tmem_load16(acc + r0, v);
+        if (swiglu) {
+          // lanes 0-15 hold gate columns, 16-31 the up columns of the same outputs: lanes below 16 take rows 0-7 of the
+          // pass, the others rows 8-15
+          const bool low = lane < 16;
+          float w[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float got = __shfl_xor_sync(0xFFFFFFFFu, low ? v[1][j] : v[0][j], 16);
+            w[j] = pf_swiglu(low ? v[0][j] : got, low ? got : v[1][j], p.limit);
+          }
+          store8(w, r0 + (low ? 0 : 8));
+        } else {
+          if (p.epi == 1) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float u = fmaxf(pf_bf16r(v[j >> 3][j & 7]), 0.f);
+              v[j >> 3][j & 7] = u * u;
+            }
+          }
+          store8(v[0], r0);
+          if (r0 + 8 < rows_here) store8(v[1], r0 + 8);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty + ab);
+      if (lane == 0) arrive_first(acc_empty0 + 8 * ab);
     }
   }
 
+  // Neither block leaves (its tensor memory, shared memory and barriers stay in use) before both are done.
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PF_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PF_TMEM_COLS) : "memory");
   }
 }
 
@@ -498,40 +593,74 @@ EncodeTiled encode_fn() {
 
 }  // namespace
 
-// dst[pos, :] = src[row(members[pos]), :]: the rows of a grouped call in member order, so an item's rows are contiguous
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, int64_t ld, const int* __restrict__ members,
-                                   const int* __restrict__ counts_total, int slots, int pairs, int k,
-                                   __nv_bfloat16* __restrict__ dst) {
-  const int lane = threadIdx.x & 31;
-  const int pos = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (pos >= pairs) return;
-  const int pair = members[pos];
-  if (pair < 0 || pair >= pairs) return;                     // members past the planned pairs hold no pair
-  const int64_t row = slots > 0 ? pair / slots : pair;
-  const uint4* s4 = reinterpret_cast<const uint4*>(src + row * ld);
-  uint4* d4 = reinterpret_cast<uint4*>(dst + static_cast<int64_t>(pos) * k);
-  for (int i = lane; i < k / 8; i += 32) d4[i] = s4[i];
+namespace {
+
+int g_pairs[64] = {};              // clusters of the prefill kernel a device runs at once (set by prefill_configure)
+
+template <int GS>
+cudaError_t launch_pairs(const CUtensorMap& map, const PrefillParams& p, int clusters, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * clusters);
+  cfg.blockDim = dim3(PF_THREADS);
+  cfg.dynamicSmemBytes = PF_SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2, attrs[0].val.clusterDim.y = 1, attrs[0].val.clusterDim.z = 1;
+  // the next kernel's blocks may take an SM as soon as this one's last wave leaves it: their weights stream while it drains
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, prefill_kernel<GS>, map, p);
 }
 
+template <int GS>
+cudaError_t configure_pairs(int* clusters) {
+  cudaError_t e = cudaFuncSetAttribute(prefill_kernel<GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(PF_THREADS);
+  cfg.dynamicSmemBytes = PF_SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(clusters, prefill_kernel<GS>, &cfg);
+}
 
-// SMs of the current device (cached per device)
-int sm_count() {
-  static int cached[64] = {};
+// Rows of a tile for an (n, m) call: the fewest cycles, waves of tiles times a tile's pace.  A stage of 64 inputs takes
+// 2 rows cycles of math, but no less than the conversion of its weights (PF_CONVERT cycles); ties go to the larger tile,
+// which converts the weights fewer times.
+constexpr int PF_CONVERT = 240;
+int pf_rows(int n, int m, int clusters) {
+  const int64_t ncp = (n + 2 * PF_COLS - 1) / (2 * PF_COLS);
+  int best = 16;
+  int64_t cost = INT64_MAX;
+  for (int rows = 16; rows <= PF_ROWS; rows += 16) {
+    const int64_t waves = (ncp * ((m + rows - 1) / rows) + clusters - 1) / clusters;
+    const int64_t c = waves * (2 * rows > PF_CONVERT ? 2 * rows : PF_CONVERT);
+    if (c <= cost) cost = c, best = rows;
+  }
+  return best;
+}
+
+int resident_pairs() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    cached[dev] = n;
-  }
-  return cached[dev];
+  return g_pairs[dev];
 }
 
-cudaError_t prefill_configure() {
-  cudaError_t e = cudaFuncSetAttribute(prefill_kernel<64, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfGeo<256>::SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_kernel<32, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfGeo<256>::SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_kernel<64, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfGeo<128>::SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_kernel<32, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfGeo<128>::SMEM);
+}  // namespace
+
+cudaError_t prefill_configure(int device) {
+  int a = 0, b = 0;
+  cudaError_t e = configure_pairs<64>(&a);
+  if (e == cudaSuccess) e = configure_pairs<32>(&b);
+  if (e == cudaSuccess && (a < 1 || b < 1)) e = cudaErrorLaunchOutOfResources;
+  if (e == cudaSuccess && device >= 0 && device < 64) g_pairs[device] = a < b ? a : b;
   return e;
 }
 
@@ -540,7 +669,7 @@ int encode_rows(CUtensorMap* map, const void* x, int64_t ldx, int rows, int k, i
   if (encode == nullptr) return fail_moe(TF_ERR_UNSUPPORTED, "prefill: the driver does not export cuTensorMapEncodeTiled");
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldx) * 2};
-  const cuuint32_t box[2] = {PF_STAGE_K, static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -570,64 +699,113 @@ extern "C" int tf_qmm_prefill_act(const void* x, int64_t ldx, int m, const void*
   if (reinterpret_cast<uintptr_t>(tiled) % 16) return fail_moe(TF_ERR_ALIGN, "tf_qmm_prefill: tiled weights must be 16-byte aligned");
   int* err = device_error_word();
   if (err == nullptr) return fail_moe(TF_ERR_STATE, "tf_qmm_prefill: tf_init has not been called for the current device");
-  CUtensorMap map;
-  if (int rc = encode_rows(&map, x, ldx, m, k, 256)) return rc;
+  const int clusters = resident_pairs();
+  if (clusters < 1) return fail_moe(TF_ERR_STATE, "tf_qmm_prefill: tf_init has not been called for the current device");
   PrefillParams p = {};
+  p.rows = pf_rows(n, m, clusters);
+  p.acc_cols = p.rows > 128 ? 192 : 128;
+  CUtensorMap map;
+  if (int rc = encode_rows(&map, x, ldx, m, k, p.rows / 2)) return rc;
   p.w = static_cast<const uint32_t*>(tiled);
   p.sb_stride = sb_stride > 0 ? sb_stride : static_cast<int64_t>(k / gs) * unit_words(4, gs);
   p.N = n, p.K = k, p.M = m;
   p.out = out, p.ldo = ldo, p.out_f32 = out_f32;
   p.err = err;
   p.epi = epi, p.limit = limit;
-  const int64_t tiles = static_cast<int64_t>((n + PF_COLS - 1) / PF_COLS) * ((m + 255) / 256);
+  const int64_t tiles = static_cast<int64_t>((n + 2 * PF_COLS - 1) / (2 * PF_COLS)) * ((m + p.rows - 1) / p.rows);
   if (tiles > (1 << 24)) return fail_moe(TF_ERR_ARG, "tf_qmm_prefill: too many tiles");
-  const int sms = sm_count();
-  if (sms < 1) return fail_moe(TF_ERR_STATE, "tf_qmm_prefill: cannot read the SM count");
-  dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));
+  const int grid = static_cast<int>(tiles < clusters ? tiles : clusters);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (gs == 64) prefill_kernel<64, 256><<<grid, PF_THREADS, PfGeo<256>::SMEM, s>>>(map, p);
-  else prefill_kernel<32, 256><<<grid, PF_THREADS, PfGeo<256>::SMEM, s>>>(map, p);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = gs == 64 ? launch_pairs<64>(map, p, grid, s) : launch_pairs<32>(map, p, grid, s);
   return e == cudaSuccess ? TF_OK : cuda_fail_moe(e, "tf_qmm_prefill");
 }
 
-extern "C" int tf_moe_experts_prefill(const void* x, int64_t ldx, int slots, const void* tiled, int64_t expert_stride,
-                                      int experts, int n, int k, int gs, const int* items, const int* counts,
-                                      const int* members, int pairs, int max_items, void* sorted, void* out, int64_t ldo,
-                                      int out_f32, int epi, float limit, void* stream) {
+namespace tf {
+namespace {
+
+// dst[pos, :] = src[row(members[pos]), :] for every planned pair: the rows of a grouped call in member order, so an item's
+// rows are contiguous.  A warp a row, four 16-byte copies in flight a lane: bound by the writes (66 MB for 12288 pairs of
+// 2688: 14 us).  Fetching the rows inside the matmul with gather copies of four rows was slower by far (a copy that is
+// not the same in every lane costs about 100 cycles to issue, 25 of them a stage).
+__global__ void __launch_bounds__(256) gather_rows_kernel(const __nv_bfloat16* __restrict__ src, int64_t ld, const int* __restrict__ items,
+                                                          const int* __restrict__ counts, const int* __restrict__ members, int slots,
+                                                          int pairs, int k, __nv_bfloat16* __restrict__ dst) {
+  const int lane = threadIdx.x & 31, pos = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int n = counts[0];
+  if (n < 1 || pos >= min(pairs, items[3 * n - 2] + items[3 * n - 1])) return;        // (past the last item: not planned)
+  const int pair = members[pos];
+  if (pair < 0 || pair >= pairs) return;
+  const int64_t row = slots > 0 ? pair / slots : pair;
+  const uint4* s4 = reinterpret_cast<const uint4*>(src + row * ld);
+  uint4* d4 = reinterpret_cast<uint4*>(dst + static_cast<int64_t>(pos) * k);
+  const int chunks = k / 8;
+  for (int i = lane; i < chunks; i += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i + 32 * j < chunks) v[j] = s4[i + 32 * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i + 32 * j < chunks) d4[i + 32 * j] = v[j];
+  }
+}
+
+}  // namespace
+}  // namespace tf
+
+extern "C" int tf_moe_gather(const void* x, int64_t ldx, int slots, const int* items, const int* counts, const int* members, int pairs,
+                             int k, void* sorted, void* stream) {
+  if (!x || !items || !counts || !members || !sorted || slots < 0 || pairs < 1 || k < 8 || k % 8 || ldx < k)
+    return fail_moe(TF_ERR_ARG, "tf_moe_gather: null pointer or bad sizes");
+  if (reinterpret_cast<uintptr_t>(x) % 16 || ldx % 8 || reinterpret_cast<uintptr_t>(sorted) % 16)
+    return fail_moe(TF_ERR_ALIGN, "tf_moe_gather: rows must start on 16-byte boundaries");
+  gather_rows_kernel<<<(pairs + 7) / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(x), ldx, items, counts, members, slots, pairs, k, static_cast<__nv_bfloat16*>(sorted));
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? TF_OK : cuda_fail_moe(e, "tf_moe_gather");
+}
+
+extern "C" int tf_moe_experts_sorted(const void* sorted, int64_t ldx, const void* tiled, int64_t expert_stride, int experts, int n, int k,
+                                     int gs, const int* items, const int* counts, const int* members, int pairs, int max_items, void* out,
+                                     int64_t ldo, int out_f32, int epi, float limit, void* stream) {
   if (experts < 1) return fail_moe(TF_ERR_ARG, "tf_moe_experts_prefill: the table holds at least one expert");
   if (gs != 32 && gs != 64) return fail_moe(TF_ERR_UNSUPPORTED, "tf_moe_experts_prefill: 4-bit weights with groups of 32 or 64");
   if (n < 1 || k < gs || k % gs || k % 8 || pairs < 1 || max_items < 1 || max_items > 65535)
     return fail_moe(TF_ERR_ARG, "tf_moe_experts_prefill: bad sizes");
   if (epi < 0 || epi > 2 || (epi == 2 && n % 32) || (epi != 0 && out_f32)) return fail_moe(TF_ERR_ARG, "tf_moe_experts_prefill: bad epilogue");
-  const int ncols = epi == 2 ? n / 2 : n;
-  if (!x || !tiled || !items || !counts || !members || !sorted || !out || ldo < ncols || slots < 0 || ldx < k)
+  if (!sorted || !tiled || !items || !counts || !out || ldo < (epi == 2 ? n / 2 : n) || ldx < k)
     return fail_moe(TF_ERR_ARG, "tf_moe_experts_prefill: null pointer or short rows");
-  if (reinterpret_cast<uintptr_t>(x) % 16 || ldx % 8 || reinterpret_cast<uintptr_t>(sorted) % 16)
-    return fail_moe(TF_ERR_ALIGN, "tf_moe_experts_prefill: rows must start on 16-byte boundaries");
+  if (reinterpret_cast<uintptr_t>(sorted) % 16 || ldx % 8 || reinterpret_cast<uintptr_t>(tiled) % 16)
+    return fail_moe(TF_ERR_ALIGN, "tf_moe_experts_prefill: rows and units must start on 16-byte boundaries");
   int* err = device_error_word();
-  if (err == nullptr) return fail_moe(TF_ERR_STATE, "tf_moe_experts_prefill: tf_init has not been called for the current device");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  gather_rows_kernel<<<(pairs + 7) / 8, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), ldx, members, counts, slots, pairs, k,
-                                                   static_cast<__nv_bfloat16*>(sorted));
+  const int clusters = resident_pairs();
+  if (err == nullptr || clusters < 1) return fail_moe(TF_ERR_STATE, "tf_moe_experts_prefill: tf_init has not been called for the current device");
   CUtensorMap map;
-  if (int rc = encode_rows(&map, sorted, k, pairs, k, 128)) return rc;
+  if (int rc = encode_rows(&map, sorted, ldx, pairs, k, PF_GROUP_ROWS / 2)) return rc;
   PrefillParams p = {};
   p.w = static_cast<const uint32_t*>(tiled);
   p.sb_stride = static_cast<int64_t>(k / gs) * unit_words(4, gs);
   p.N = n, p.K = k, p.M = pairs;
+  p.rows = p.acc_cols = PF_GROUP_ROWS;
   p.out = out, p.ldo = ldo, p.out_f32 = out_f32;
   p.err = err;
   p.items = items, p.counts = counts, p.members = members;
   p.expert_stride = expert_stride;
   p.experts = experts;
   p.epi = epi, p.limit = limit;
-  const int64_t tiles = static_cast<int64_t>((n + PF_COLS - 1) / PF_COLS) * max_items;   // upper bound: the plan says how many
-  const int sms = sm_count();
-  if (sms < 1) return fail_moe(TF_ERR_STATE, "tf_moe_experts_prefill: cannot read the SM count");
-  dim3 grid(static_cast<unsigned>(tiles < sms ? tiles : sms));
-  if (gs == 64) prefill_kernel<64, 128><<<grid, PF_THREADS, PfGeo<128>::SMEM, s>>>(map, p);
-  else prefill_kernel<32, 128><<<grid, PF_THREADS, PfGeo<128>::SMEM, s>>>(map, p);
-  const cudaError_t e = cudaGetLastError();
+  const int64_t tiles = static_cast<int64_t>((n + 2 * PF_COLS - 1) / (2 * PF_COLS)) * max_items;   // upper bound: the plan says how many
+  const int grid = static_cast<int>(tiles < clusters ? tiles : clusters);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = gs == 64 ? launch_pairs<64>(map, p, grid, s) : launch_pairs<32>(map, p, grid, s);
   return e == cudaSuccess ? TF_OK : cuda_fail_moe(e, "tf_moe_experts_prefill");
+}
+
+extern "C" int tf_moe_experts_prefill(const void* x, int64_t ldx, int slots, const void* tiled, int64_t expert_stride,
+                                      int experts, int n, int k, int gs, const int* items, const int* counts,
+                                      const int* members, int pairs, int max_items, void* sorted, void* out, int64_t ldo,
+                                      int out_f32, int epi, float limit, void* stream) {
+  if (!members) return fail_moe(TF_ERR_ARG, "tf_moe_experts_prefill: null pointer");
+  if (int rc = tf_moe_gather(x, ldx, slots, items, counts, members, pairs, k, sorted, stream)) return rc;
+  return tf_moe_experts_sorted(sorted, k, tiled, expert_stride, experts, n, k, gs, items, counts, members, pairs, max_items, out, ldo,
+                               out_f32, epi, limit, stream);
 }

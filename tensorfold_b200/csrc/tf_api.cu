@@ -57,7 +57,7 @@ std::mutex g_init_mutex;
 
 }  // namespace
 
-cudaError_t prefill_configure();      // qmm_prefill.cu
+cudaError_t prefill_configure(int device);      // qmm_prefill.cu
 void peer_reduce_plain(int on);       // peer_reduce.cu
 cudaError_t moe_static_init(int device);   // moe.cu: the built-in plan scratch's address on that device
 int encode_rows(CUtensorMap* map, const void* x, int64_t ldx, int rows, int k, int box_rows);
@@ -278,7 +278,7 @@ int tf_init(int device) {
   if (e == cudaSuccess) e = qmm_configure_b5();
   if (e == cudaSuccess) e = qmm_configure_b6();
   if (e == cudaSuccess) e = qmm_configure_b8();
-  if (e == cudaSuccess) e = prefill_configure();
+  if (e == cudaSuccess) e = prefill_configure(device);
   if (e == cudaSuccess) e = qmm_stream_configure_b2();
   if (e == cudaSuccess) e = qmm_stream_configure_b3();
   if (e == cudaSuccess) e = qmm_stream_configure_b4();

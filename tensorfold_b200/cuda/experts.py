@@ -162,18 +162,29 @@ def _grouped(x, slots, table, n, k, ex, plan, out, rows, epi, limit):
     stream = _lib.stream_of(x)
     items = min(max_items(rows * plan.slots, plan.experts, plan.tile), plan.items.shape[0])
     if plan.prefill:
-        if ex.gs not in (32, 64):
-            raise ValueError("prefill plans take expert weights with groups of 32 or 64")
-        pairs = plan.members.shape[0]
-        if plan.sorted is None or plan.sorted.numel() < pairs * k:
-            plan.sorted = torch.empty((pairs * max(k, ex.dims, ex.width),), dtype=torch.bfloat16, device=x.device)
+        _prefill_format(ex)
         _lib.native().tf_moe_experts_prefill(
             "experts (prefill)", x, x.stride(0), slots, table, table.stride(0), table.shape[0], n, k, ex.gs, plan.items, plan.counts,
-            plan.members, rows * plan.slots, items, plan.sorted, out, out.stride(0), out.dtype == torch.float32, epi, limit, stream)
+            plan.members, rows * plan.slots, items, _sorted(plan, ex, x), out, out.stride(0), out.dtype == torch.float32, epi, limit,
+            stream)
         return
     _lib.native().tf_moe_experts(
         "experts", x, x.stride(0), slots, table, table.stride(0), table.shape[0], n, k, ex.gs, plan.items, plan.counts, plan.members,
         items, plan.tile, out, out.stride(0), out.dtype == torch.float32, epi, limit, stream)
+
+
+def _prefill_format(ex: Experts) -> None:
+    if ex.gs not in (32, 64):
+        raise ValueError("prefill plans take expert weights with groups of 32 or 64")
+
+
+def _sorted(plan: Plan, ex: Experts, x: torch.Tensor) -> torch.Tensor:
+    """Scratch for a call's rows in member order, made on first use."""
+
+    need = plan.members.shape[0] * max(ex.dims, ex.width)
+    if plan.sorted is None or plan.sorted.numel() < need:
+        plan.sorted = torch.empty((need,), dtype=torch.bfloat16, device=x.device)
+    return plan.sorted
 
 
 def gate_up(x: torch.Tensor, ex: Experts, plan: Plan, out: torch.Tensor, rows: int) -> None:
@@ -191,3 +202,27 @@ def down(act: torch.Tensor, ex: Experts, plan: Plan, out: torch.Tensor, rows: in
     if out.dtype not in (torch.float32, torch.bfloat16) or out.shape[1] != ex.dims:
         raise ValueError("down: out must be (pairs, D) fp32 or bf16")
     _grouped(act, 0, ex.down, ex.dims, ex.width, ex, plan, out, rows, 0, 0.0)
+
+
+def layer(x: torch.Tensor, ex: Experts, plan: Plan, act: torch.Tensor, out: torch.Tensor, rows: int) -> None:
+    """``gate_up`` into ``act`` [R * slots, NI], then ``down`` into ``out`` [R * slots, D].  In the prefill form ``act`` holds the
+    activations in member order, so that ``down`` reads an expert's rows where they are; ``out`` is the same."""
+
+    if not plan.prefill or plan.experts > ex.count or x.dim() != 2 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+        gate_up(x, ex, plan, act, rows)
+        down(act, ex, plan, out, rows)
+        return
+    if act.dtype != torch.bfloat16 or act.shape[1] != ex.width or x.dtype != torch.bfloat16 or x.shape[1] != ex.dims:
+        raise ValueError(f"experts: x must be (rows, {ex.dims}) and act (pairs, {ex.width}), both bf16")
+    if out.dtype not in (torch.float32, torch.bfloat16) or out.dim() != 2 or out.shape[1] != ex.dims or out.stride(1) != 1:
+        raise ValueError("experts: out must be (pairs, D) fp32 or bf16 with unit-stride rows")
+    _prefill_format(ex)
+    lib, stream, pairs, rows_in = _lib.native(), _lib.stream_of(x), rows * plan.slots, _sorted(plan, ex, x)
+    items = min(max_items(pairs, plan.experts, plan.tile), plan.items.shape[0])
+    lib.tf_moe_gather("experts (gather)", x, x.stride(0), plan.slots, plan.items, plan.counts, plan.members, pairs, ex.dims, rows_in, stream)
+    lib.tf_moe_experts_sorted("experts (gate, up)", rows_in, ex.dims, ex.up, ex.up.stride(0), ex.count, (2 if ex.swiglu else 1) * ex.width,
+                              ex.dims, ex.gs, plan.items, plan.counts, None, pairs, items, act, act.stride(0), 0, 2 if ex.swiglu else 1,
+                              ex.limit, stream)
+    lib.tf_moe_experts_sorted("experts (down)", act, act.stride(0), ex.down, ex.down.stride(0), ex.count, ex.dims, ex.width, ex.gs,
+                              plan.items, plan.counts, plan.members, pairs, items, out, out.stride(0), out.dtype == torch.float32, 0, 0.0,
+                              stream)

@@ -95,8 +95,7 @@ def moe(x: torch.Tensor, router_rows: torch.Tensor, ex: grouped.Experts, buf: Mo
     def routed() -> None:
         router(x, router_rows, buf.logits[:rows], prefill=buf.plan.prefill)
         select(buf.logits[:rows], buf, top_k, experts)
-        grouped.gate_up(x, ex, buf.plan, buf.act.view(-1, ex.width), rows)
-        grouped.down(buf.act.view(-1, ex.width), ex, buf.plan, buf.y.view(-1, ex.dims), rows)
+        grouped.layer(x, ex, buf.plan, buf.act.view(-1, ex.width), buf.y.view(-1, ex.dims), rows)
 
     def dense() -> None:
         if buf.plan.prefill:                                    # prefill arithmetic for the dense shared expert too

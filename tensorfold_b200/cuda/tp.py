@@ -207,8 +207,7 @@ class ExpertParallelMoE:
         moe.select_local_rows(logits, buf, self.top_k, self.total, self.first, self.experts.count)
         wts = buf.wts[:rows]
         grouped.route(buf.pick[:rows], buf.plan)
-        grouped.gate_up(x, self.experts, buf.plan, buf.act.view(-1, self.experts.width), rows)
-        grouped.down(buf.act.view(-1, self.experts.width), self.experts, buf.plan, buf.y.view(-1, self.experts.dims), rows)
+        grouped.layer(x, self.experts, buf.plan, buf.act.view(-1, self.experts.width), buf.y.view(-1, self.experts.dims), rows)
         return moe.combine(buf.y[:rows], wts, out)
 
     def run(self, x: torch.Tensor, buf: moe.MoEBuffers, group=None, reducer: PeerReducer | None = None) -> torch.Tensor:

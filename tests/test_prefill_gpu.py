@@ -39,6 +39,44 @@ def test_matches_the_oracle(n, k, gs, m):
     assert _lib.device_error(y) == 0
 
 
+@pytest.mark.parametrize("n,k,gs,m", [(1, 64, 64, 17), (136, 192, 64, 193), (257, 128, 64, 385), (392, 320, 32, 16), (1160, 704, 64, 130)])
+def test_edges_of_the_paired_tiles(n, k, gs, m):
+    """Columns past one block of a pair and past 8, an odd number of 128-column blocks, rows one past a tile of 16, 128 or
+    192, and K that ends with half of a 128-input stage; the oracle and the tolerance of the test above."""
+
+    w = synthetic.affine_weight(n, k, 4, gs, seed=n + m)
+    q = qmm.pack(*to_dev(*w), gs)
+    x = synthetic.activations(m, k, 4)
+    ref = reference(x, *w, gs)
+    f32 = qmm.prefill_matmul(x.to(DEV), q, f32=True)
+    assert np.abs(f32.cpu().numpy() - ref).max() <= np.abs(ref).max() * 2 ** -12
+    wide = torch.full((m, n + 8), 7.0, dtype=torch.bfloat16, device=DEV)                  # a slice of wider rows as output
+    y = qmm.prefill_matmul(x.to(DEV), q, out=wide[:, :n])
+    assert torch.equal(y, f32.to(torch.bfloat16)) and bool((wide[:, n:] == 7.0).all())
+    assert _lib.device_error(y) == 0
+
+
+@pytest.mark.parametrize("act", ["swiglu", "relu2"])
+@pytest.mark.parametrize("k,m", [(96, 33), (160, 200)])
+def test_epilogues_at_the_edges(act, k, m):
+    """K ends inside a half stage (groups of 32); the epilogue works on the bf16 of the plain product's sums."""
+
+    gs, half = 32, 144
+    a, b = (synthetic.affine_weight(half, k, 4, gs, seed=s) for s in (5, 6))
+    q = qmm.pack_pair(to_dev(*a), to_dev(*b), gs)
+    x = synthetic.activations(m, k, 8).to(DEV)
+    got = qmm.matmul_act(x, q, act=act, prefill=True).float()
+    v = torch.from_numpy(np.concatenate([reference(x.cpu(), *w, gs) for w in (a, b)], 1)).to(torch.bfloat16).double()
+    gate, up = v[:, :half], v[:, half:]
+    if act == "swiglu":
+        want = (gate / (1 + torch.exp(-gate))).to(torch.bfloat16).double() * up
+    else:
+        want = torch.stack([gate.view(m, 9, 16), up.view(m, 9, 16)], 2).view(m, 2 * half).clamp(min=0) ** 2
+    # a factor may round to the neighbouring bf16 value (2^-8 relative each), the product rounds once more
+    assert (got.cpu().double() - want).abs().max() <= want.abs().max() * 3 * 2 ** -8
+    assert _lib.device_error(x) == 0
+
+
 def test_exact_integer_case_is_bit_exact():
     rng = np.random.default_rng(7)
     n, k, gs, m = 140, 128, 64, 19
