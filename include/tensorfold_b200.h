@@ -106,6 +106,17 @@ int tf_qmm(const void* x, int64_t ldx, int m, const float* xs, const void* tiled
            int bits, int gs, int sk, void* out, int64_t ldo, int out_f32, float* part, int reduce, int pdl,
            void* stream);
 
+/* tf_qmm for 17 and more rows (any number works) on the tcgen05 kernel: the bits of tf_qmm with reduce = 1.  Codes of 2, 3,
+ * 4, 5 or 6 bits.
+ *   scratch  with sk > 1: 64 KB of counters, 256-byte aligned, zero before the first call and left zero by every call;
+ *            two launches that share it must not overlap
+ *   part     with sk > 1: tf_qmm_window_part_bytes(m, n, bits, sk) bytes, 16-byte aligned, contents free
+ * tf_qmm_window_part_bytes is negative where the kernel does not take the call. */
+int64_t tf_qmm_window_part_bytes(int m, int n, int bits, int sk);
+int tf_qmm_window(const void* x, int64_t ldx, int m, const float* xs, const void* tiled, int64_t sb_stride, int n, int k,
+                  int bits, int gs, int sk, void* out, int64_t ldo, int out_f32, void* scratch, int64_t scratch_bytes,
+                  float* part, int64_t part_bytes, int pdl, void* stream);
+
 /* tf_qmm for decode and verify windows (1 to 16 rows) over a SET of up to 4 projections that read the same rows of x
  * (q/k/v, gate/up, or one projection alone): one persistent launch streams all of them, and every output row has the
  * bits tf_qmm gives for the same projection and slice count.  Host arrays of nproj entries: tiled, sb_stride (entries

@@ -31,6 +31,9 @@ SIGNATURES = {
     "tf_group_sums": (_i32, (_vp, _i64, _i32, _i32, _i32, _vp, _vp)),
     "tf_qmm": (_i32, (_vp, _i64, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _i32, _vp, _i32, _i32,
                       _vp)),
+    "tf_qmm_window_part_bytes": (_i64, (_i32, _i32, _i32, _i32)),
+    "tf_qmm_window": (_i32, (_vp, _i64, _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _i32, _vp, _i64, _vp, _i64,
+                             _i32, _vp)),
     "tf_qmm_set_scratch_bytes": (_i64, (_i32, _vp, _vp)),
     "tf_qmm_set_geometry": (_i32, (_i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp)),
     "tf_qmm_set": (_i32, (_vp, _i64, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _i64, _i32,

@@ -10,6 +10,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
@@ -29,7 +30,7 @@ namespace {
 // the library's entry points
 // ---------------------------------------------------------------------------------------------------------------------
 
-#define TF_WRAPPED(X) X(tf_qmm) X(tf_qmm_set) X(tf_qmm_set_scratch_bytes) X(tf_qmm_prefill) X(tf_qmm_prefill_act) X(tf_qmm_act) \
+#define TF_WRAPPED(X) X(tf_qmm) X(tf_qmm_set) X(tf_qmm_set_scratch_bytes) X(tf_qmm_window) X(tf_qmm_window_part_bytes) X(tf_qmm_prefill) X(tf_qmm_prefill_act) X(tf_qmm_act) \
   X(tf_add_rmsnorm) X(tf_swiglu)
 #define TF_THUNKS(X) X(tf_pack) X(tf_pack_pair) X(tf_unpack) X(tf_group_sums) X(tf_affine_rows) X(tf_moe_plan) X(tf_moe_experts) \
   X(tf_moe_experts_prefill) X(tf_moe_gather) X(tf_moe_experts_sorted) X(tf_moe_router) X(tf_moe_router_tiles) X(tf_moe_topk) X(tf_moe_topk_local) X(tf_moe_combine)
@@ -244,6 +245,52 @@ void run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
         who);
 }
 
+// Which of the two kernels for more than 16 rows (their bits are the same).  The tensor-memory kernel works on one block an
+// SM and its roles start one after another, about 4 us that the tiled kernel does not pay; that kernel in turn repeats its
+// conversion and its mma.sync for every 64 rows.  Measured at 4 bits, groups of 64, in us (tensor memory / tiled):
+// 17408 x 5120 36 / 31 at 17 rows, 37 / 33 at 32, 38 / 66 at 48, 142 / 254 at 256; 4096 x 4096 30 / 35 at 48; below the
+// line 1024 x 5120 22 / 18 at 64 and 128, above it 23 / 31 at 256; 256 x 512 12 / 8 at 17 to 256; 6 bits in groups of 128,
+// 2048 x 4096 21 / 17 at 64, 19 / 29 at 96.
+bool window_pays(int64_t m, const Weight& q) {
+  return m > 32 && (m + 63) / 64 * q.n * q.k >= (int64_t{1} << 24);
+}
+
+// The counters of the tensor-memory kernel's slices: zero, and left zero by every launch.  An eager call uses its stream's
+// own 64 KB (made once a stream, returned by reset_scratch); a captured call, whose graph may be replayed beside another
+// graph captured on the same stream, gets counters that belong to the graph and are zeroed in it.
+constexpr int64_t COUNTER_BYTES = 64 * 1024;
+auto& g_counters = *new std::map<std::pair<int, cudaStream_t>, at::Tensor>;      // (outlives the allocator's tear-down)
+
+at::Tensor counters_of(const at::Tensor& x, cudaStream_t stream) {
+  const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  const auto key = std::make_pair(static_cast<int>(x.get_device()), stream);
+  if (!capturing) {
+    const auto hit = g_counters.find(key);
+    if (hit != g_counters.end()) return hit->second;
+  }
+  at::Tensor made = empty({COUNTER_BYTES}, at::kByte, x);
+  made.zero_();
+  if (!capturing && g_counters.size() < 256) g_counters[key] = made;
+  return made;
+}
+
+// matmul on the tensor-memory kernel.  False: the call is not one for it (8-bit codes, too many columns for its counters).
+bool run_window(const at::Tensor& x, const Weight& q, int sk, const float* sums, bool f32, const at::Tensor& out, bool pdl,
+                cudaStream_t stream, const char* who) {
+  const int m = static_cast<int>(x.size(0));
+  const int64_t need = p_tf_qmm_window_part_bytes(m, q.n, q.bits, sk);
+  if (need < 0 || static_cast<int64_t>(sk) * (q.k / q.gs) > (1 << 30)) return false;
+  at::Tensor part, counters;
+  if (sk > 1) part = empty({need / 4}, at::kFloat, x), counters = counters_of(x, stream);
+  check(unlocked([&] {
+          return p_tf_qmm_window(x.data_ptr(), x.stride(0), m, sums, q.units.data_ptr(), q.units.stride(0), q.n, q.k, q.bits, q.gs, sk,
+                                 out.data_ptr(), out.stride(0), f32, counters.defined() ? counters.data_ptr() : nullptr, COUNTER_BYTES,
+                                 part.defined() ? part.data_ptr<float>() : nullptr, need, pdl, stream);
+        }),
+        who);
+  return true;
+}
+
 // matmul(x, q, xs, sk, f32, out, part, reduce, pdl, stream)
 PyObject* matmul(PyObject* const* a) {
   const char* who = "matmul";
@@ -263,6 +310,8 @@ PyObject* matmul(PyObject* const* a) {
     return THPVariable_Wrap(out);
   }
   const float* sums = sums_of(a[2], m, kg, who);
+  if (truth(a[9]) && window_pays(m, q) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))
+    return THPVariable_Wrap(out);
   at::Tensor part;
   if (sk > 1 && (!reduce || sk > 8)) {
     if (a[6] == Py_None) {
@@ -494,6 +543,7 @@ PyObject* py_stream_of(PyObject*, PyObject* t) {
 
 PyObject* py_forget_scratch(PyObject*, PyObject*) {
   g_scratch.clear();
+  g_counters.clear();
   Py_RETURN_NONE;
 }
 

@@ -11,6 +11,7 @@
 #include "../../include/tensorfold_b200.h"
 #include "qmm_launch.h"
 #include "qmm_stream_launch.h"
+#include "qmm_window_launch.h"
 
 namespace tf {
 
@@ -230,6 +231,25 @@ int64_t set_part_bytes(int n, int sk) {
   return sk > 1 ? static_cast<int64_t>((n + SB_COLS - 1) / SB_COLS) * sk * STREAM_PART_FLOATS * 4 : 0;
 }
 
+// A launch of the window kernel takes up to WINDOW_CHUNK rows in equal tiles of at most 64 (rounded up to 16).
+constexpr int WINDOW_CHUNK = 256;
+int window_tiles(int m) { return (std::min(m, WINDOW_CHUNK) + 63) / 64; }
+int window_tile_rows(int m) {
+  const int rows = std::min(m, WINDOW_CHUNK), t = window_tiles(m);
+  return ((rows + t - 1) / t + 15) / 16 * 16;
+}
+
+cudaError_t window_launch_bits(const CUtensorMap& tmx, const WindowParams& p, int bits, int gs, int rows, int grid, cudaStream_t s,
+                               bool pdl) {
+  switch (bits) {
+    case 2: return qmm_window_launch_b2(tmx, p, gs, rows, grid, s, pdl);
+    case 3: return qmm_window_launch_b3(tmx, p, gs, rows, grid, s, pdl);
+    case 4: return qmm_window_launch_b4(tmx, p, gs, rows, grid, s, pdl);
+    case 5: return qmm_window_launch_b5(tmx, p, gs, rows, grid, s, pdl);
+    default: return qmm_window_launch_b6(tmx, p, gs, rows, grid, s, pdl);
+  }
+}
+
 int grid_for(int64_t total, int threads) {
   const int64_t blocks = (total + threads - 1) / threads;
   return static_cast<int>(blocks < 1 ? 1 : (blocks > 148 * 32 ? 148 * 32 : blocks));
@@ -285,6 +305,11 @@ int tf_init(int device) {
   if (e == cudaSuccess) e = qmm_stream_configure_b5();
   if (e == cudaSuccess) e = qmm_stream_configure_b6();
   if (e == cudaSuccess) e = qmm_stream_configure_b8();
+  if (e == cudaSuccess) e = qmm_window_configure_b2();
+  if (e == cudaSuccess) e = qmm_window_configure_b3();
+  if (e == cudaSuccess) e = qmm_window_configure_b4();
+  if (e == cudaSuccess) e = qmm_window_configure_b5();
+  if (e == cudaSuccess) e = qmm_window_configure_b6();
   int sms = 0;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) {
@@ -541,6 +566,57 @@ int tf_qmm_set(const void* x, int64_t ldx, int m, const float* xs, int k, int bi
   const int grid = std::min(items, st->sms * resident);
   const cudaError_t e = stream_launch_bits(tmx, p, bits, gs, mt, kw, grid, static_cast<cudaStream_t>(stream), pdl != 0);
   return e == cudaSuccess ? TF_OK : cuda_fail(e, "tf_qmm_set launch");
+}
+
+int64_t tf_qmm_window_part_bytes(int m, int n, int bits, int sk) {
+  if (m < 1 || m > 65535 * 8 || n < 1 || sk < 1 || sk > 32767 || bits == 8) return TF_ERR_UNSUPPORTED;
+  if (sk == 1) return 0;
+  const int64_t quads = static_cast<int64_t>(window_tiles(m)) * ((n + SB_COLS - 1) / SB_COLS);
+  if (quads * 16 > SET_COUNTER_BYTES) return TF_ERR_UNSUPPORTED;      // its counters: as many bytes as a set's
+  return quads * sk * (SB_COLS * 4) * window_rows(window_tile_rows(m));
+}
+
+int tf_qmm_window(const void* x, int64_t ldx, int m, const float* xs, const void* tiled, int64_t sb_stride, int n, int k, int bits,
+                  int gs, int sk, void* out, int64_t ldo, int out_f32, void* scratch, int64_t scratch_bytes, float* part,
+                  int64_t part_bytes, int pdl, void* stream) {
+  if (!format_ok(bits, gs) || bits == 8) return fail(TF_ERR_ARG, "tf_qmm_window: %d bits / groups of %d", bits, gs);
+  if (m < 1 || n < 1 || k < gs || k % gs) return fail(TF_ERR_ARG, "tf_qmm_window: bad shape m=%d n=%d k=%d", m, n, k);
+  const int kg = k / gs;
+  if (sk < 1 || sk > kg) return fail(TF_ERR_ARG, "tf_qmm_window: 1 to %d K slices (one group at least a slice), not %d", kg, sk);
+  if (!x || !tiled || !out || ldo < n || sb_stride < 0) return fail(TF_ERR_ARG, "tf_qmm_window: null pointer, short out rows or a negative stride");
+  if (reinterpret_cast<uintptr_t>(x) % 16 || (m > 1 && ldx % 8) || ldx < k)
+    return fail(TF_ERR_ALIGN, "tf_qmm_window: x rows must start on 16-byte boundaries (ldx %% 8 == 0, ldx >= k)");
+  if (reinterpret_cast<uintptr_t>(tiled) % 16) return fail(TF_ERR_ALIGN, "tf_qmm_window: tiled weights must be 16-byte aligned");
+  if (static_cast<int64_t>(sk) * kg + kg > 0x7fffffff) return fail(TF_ERR_ARG, "tf_qmm_window: K is too long");
+  const int64_t need = tf_qmm_window_part_bytes(m, n, bits, sk);
+  if (need < 0) return fail(TF_ERR_ARG, "tf_qmm_window: too many rows, slices or columns");
+  if (sk > 1 && (!scratch || reinterpret_cast<uintptr_t>(scratch) % 256 || scratch_bytes < SET_COUNTER_BYTES || !part ||
+                 reinterpret_cast<uintptr_t>(part) % 16 || part_bytes < need))
+    return fail(TF_ERR_ARG, "tf_qmm_window: %lld bytes of zeroed counters and %lld of slices", static_cast<long long>(SET_COUNTER_BYTES),
+                static_cast<long long>(need));
+  DeviceState* st = nullptr;
+  if (int rc = current_state(&st)) return rc;
+  WindowParams p = {};
+  p.w = static_cast<const uint32_t*>(tiled);
+  p.sb_stride = sb_stride > 0 ? sb_stride : static_cast<int64_t>(kg) * unit_words(bits, gs);
+  p.ldo = ldo, p.out_f32 = out_f32, p.part = part, p.count = static_cast<int*>(scratch);
+  p.N = n, p.KG = kg, p.sk = sk, p.nsb = (n + SB_COLS - 1) / SB_COLS;
+  p.tile_rows = window_tile_rows(m);
+  p.err = st->err;
+  const int rows = window_rows(p.tile_rows);
+  for (int m0 = 0; m0 < m; m0 += WINDOW_CHUNK) {             // launches of one stream: they share counters and slices in turn
+    p.M = std::min(WINDOW_CHUNK, m - m0);
+    p.row_tiles = (p.M + p.tile_rows - 1) / p.tile_rows;
+    p.xs = xs ? xs + static_cast<int64_t>(m0) * kg : nullptr;
+    p.out = static_cast<uint8_t*>(out) + m0 * ldo * (out_f32 ? 4 : 2);
+    p.items = (p.nsb + 1) / 2 * sk * p.row_tiles;
+    CUtensorMap tmx = {};
+    if (int rc = encode_rows(&tmx, static_cast<const __nv_bfloat16*>(x) + m0 * ldx, p.M == 1 ? k : ldx, p.M, k, rows)) return rc;
+    const cudaError_t e = window_launch_bits(tmx, p, bits, gs, rows, std::min(p.items, st->sms), static_cast<cudaStream_t>(stream),
+                                             pdl != 0 && m0 == 0);
+    if (e != cudaSuccess) return cuda_fail(e, "tf_qmm_window launch");
+  }
+  return TF_OK;
 }
 
 int tf_qmm_act(const void* x, int64_t ldx, int m, const void* tiled, int64_t sb_stride, int n, int k, int bits, int gs,
