@@ -348,6 +348,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     if (!ok) let_copies_land();
   } else if (warp == 2) {
     // ------------------------------------------------------------------ packed units (HBM -> shared, bulk copies)
+    if (!grouped) pdl_wait();                                // the units may be the previous kernel's output too
     bool ok = true;
     int slot = 0;
     uint32_t phase = 1;
@@ -607,7 +608,8 @@ cudaError_t launch_pairs(const CUtensorMap& map, const PrefillParams& p, int clu
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeClusterDimension;
   attrs[0].val.clusterDim.x = 2, attrs[0].val.clusterDim.y = 1, attrs[0].val.clusterDim.z = 1;
-  // the next kernel's blocks may take an SM as soon as this one's last wave leaves it: their weights stream while it drains
+  // the next kernel's blocks may take an SM as soon as this one's last wave leaves it and set up there; they read and write
+  // global memory, weights among it, only once this one is done (the caller is not asked whether they are settled)
   attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;

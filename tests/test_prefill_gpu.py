@@ -77,6 +77,29 @@ def test_epilogues_at_the_edges(act, k, m):
     assert _lib.device_error(x) == 0
 
 
+@pytest.mark.parametrize("act", [None, "relu2"])
+def test_weights_the_previous_kernel_wrote(act):
+    """A prompt matmul writes the packed units (as bf16 rows) that the next one multiplies with, and nothing waits in
+    between: its blocks run on few SMs for long, and signal their dependents at once."""
+
+    n, kg, gs = 2048, 8, 64
+    q1 = qmm.pack(*to_dev(*synthetic.raw_weight(2304, 16384, 4, 64, 1)), 64)
+    x1 = synthetic.activations(n // 128 * kg, 16384, 2).to(DEV)
+    x2 = synthetic.activations(48, kg * gs, 3).to(DEV)
+    units = torch.zeros((n // 128, kg, 1152), dtype=torch.int32, device=DEV)
+    q2 = qmm.Q4(units, None, None, n, kg * gs, gs)
+    run = lambda: qmm.prefill_matmul(x2, q2, f32=True) if act is None else qmm.matmul_act(x2, q2, act=act, prefill=True)
+    for _ in range(3):
+        units.zero_()
+        torch.cuda.synchronize()
+        qmm.prefill_matmul(x1, q1, out=units.view(torch.bfloat16).view(-1, 2304))
+        got = run()
+        torch.cuda.synchronize()
+        want = run()
+        assert torch.isfinite(want).all() and want.any()
+        assert torch.equal(got, want)
+
+
 def test_exact_integer_case_is_bit_exact():
     rng = np.random.default_rng(7)
     n, k, gs, m = 140, 128, 64, 19
