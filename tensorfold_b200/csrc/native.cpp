@@ -197,17 +197,18 @@ int split_of(PyObject* sk, const Weight& q) {
   return value;
 }
 
+// The area is handed out as a tensor: Python may replace it (a larger set) or drop it (reset_scratch) from another thread
+// while a launch that uses it has given up the interpreter lock.
 PyObject* g_scratch_for = nullptr;        // Python: (device, stream, bytes) -> the stream's scratch area
-std::map<std::pair<int, cudaStream_t>, std::pair<void*, int64_t>> g_scratch;
+auto& g_scratch = *new std::map<std::pair<int, cudaStream_t>, at::Tensor>;       // (outlives the allocator's tear-down)
 
-std::pair<void*, int64_t> scratch_of(int dev, cudaStream_t stream, int64_t need) {
+at::Tensor scratch_of(int dev, cudaStream_t stream, int64_t need) {
   const auto key = std::make_pair(dev, stream);
   const auto hit = g_scratch.find(key);
-  if (hit != g_scratch.end() && hit->second.second >= need) return hit->second;
+  if (hit != g_scratch.end() && hit->second.numel() >= need) return hit->second;
   Owned area(PyObject_CallFunction(g_scratch_for, "iKL", dev, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)),
                                    static_cast<long long>(need)));
-  const at::Tensor& t = tensor(area.p, "scratch");          // Python keeps it alive until reset_scratch
-  return g_scratch[key] = std::make_pair(t.data_ptr(), t.numel());
+  return g_scratch[key] = tensor(area.p, "scratch");
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -235,12 +236,14 @@ void run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
   }
   const int64_t need = p_tf_qmm_set_scratch_bytes(count, n, sk);
   if (need < 0) refuse("%s: bad shapes", who);
-  const auto scratch = scratch_of(x.get_device(), stream, need);
+  const at::Tensor scratch = scratch_of(x.get_device(), stream, need);
+  void* const area = scratch.data_ptr();
+  const int64_t room = scratch.numel();
   const void* xp = x.data_ptr();
   const int64_t ldx = x.stride(0);
   check(unlocked([&] {
           return p_tf_qmm_set(xp, ldx, static_cast<int>(m), sums, k, q[0].bits, q[0].gs, count, tiled, stride, n, sk, out, ldo, f32,
-                              scratch.first, scratch.second, pdl, stream);
+                              area, room, pdl, stream);
         }),
         who);
 }
@@ -259,7 +262,7 @@ bool window_pays(int64_t m, const Weight& q) {
 // own 64 KB (made once a stream, returned by reset_scratch); a captured call, whose graph may be replayed beside another
 // graph captured on the same stream, gets counters that belong to the graph and are zeroed in it.
 constexpr int64_t COUNTER_BYTES = 64 * 1024;
-auto& g_counters = *new std::map<std::pair<int, cudaStream_t>, at::Tensor>;      // (outlives the allocator's tear-down)
+auto& g_counters = *new std::map<std::pair<int, cudaStream_t>, at::Tensor>;
 
 at::Tensor counters_of(const at::Tensor& x, cudaStream_t stream) {
   const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;

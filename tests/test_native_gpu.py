@@ -1,0 +1,54 @@
+"""The host path (``csrc/native.cpp``) on a B200: who owns the memory a launch was given."""
+
+import ctypes
+import subprocess
+
+import pytest
+import torch
+
+from tensorfold_b200 import _lib, synthetic
+from tensorfold_b200.cuda.kernels import qmm
+
+from gpu_util import DEV, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def stand_in(folder):
+    """A library with every entry point that launches nothing: they return 0, and ``tf_qmm_set`` what ``*during`` returns."""
+
+    text = "long long (*during)(void);\n" + "".join(
+        f"long long {name}() {{ return {'during()' if name == 'tf_qmm_set' else 65536 if name.endswith('_bytes') else 0}; }}\n"
+        for name in _lib.SIGNATURES)
+    (folder / "stand_in.c").write_text(text)
+    subprocess.run(["gcc", "-w", "-shared", "-fPIC", "-o", str(folder / "stand_in.so"), str(folder / "stand_in.c")], check=True)
+    return folder / "stand_in.so"
+
+
+def test_a_launch_holds_its_scratch_area(tmp_path):
+    """Another thread may drop every scratch area while a launch has given up the interpreter lock; the memory of the one in
+    use must not reach a new tensor before the call is back."""
+
+    q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 1)), 64)
+    x = synthetic.activations(4, 1024, 2).to(DEV)
+    want = qmm.matmul(x, q, sk=2)
+    area = qmm._set_scratch[x.device.index, _lib.stream_of(x)]
+    held, size, taken = area.data_ptr(), area.numel(), []
+    del area
+
+    def during():
+        qmm.reset_scratch()
+        keep = [torch.empty((size,), dtype=torch.uint8, device=DEV) for _ in range(2 * qmm.SCRATCH_AREAS)]
+        taken.extend(t.data_ptr() for t in keep)
+        return 0
+
+    path, callback = stand_in(tmp_path), ctypes.CFUNCTYPE(ctypes.c_longlong)(during)
+    ctypes.c_void_p.in_dll(ctypes.CDLL(str(path)), "during").value = ctypes.cast(callback, ctypes.c_void_p).value
+    native = _lib.native()
+    native.bind(str(path), _lib.ensure_device)
+    try:
+        qmm.matmul(x, q, sk=2)
+    finally:
+        native.bind(str(_lib.LIB_PATH), _lib.ensure_device)
+    assert taken and held not in taken
+    assert torch.equal(qmm.matmul(x, q, sk=2), want)          # a new area, zeroed
