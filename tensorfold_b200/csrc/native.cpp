@@ -216,10 +216,12 @@ at::Tensor scratch_of(int dev, cudaStream_t stream, int64_t need) {
 // ---------------------------------------------------------------------------------------------------------------------
 
 constexpr int SET_MAX = 4, SET_ROWS = 16;
+constexpr int CLUSTER_SLICES = 8;         // K slices tf_qmm adds on chip; more leave it through `part`
 
-// Projections of the same 1 to 16 rows in one persistent launch; `outs` are filled in.
-void run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyObject* xs, bool f32, at::Tensor* outs, bool pdl,
-             const char* who) {
+// Projections of the same 1 to 16 rows in one persistent launch; `outs` are filled in.  With `optional` it returns false where
+// the sets' scratch has no room for the slices and cannot be given any (a new area during a capture): nothing is launched.
+bool run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyObject* xs, bool f32, at::Tensor* outs, bool pdl,
+             const char* who, bool optional = false) {
   const cudaStream_t stream = stream_of(x);
   const int64_t m = x.size(0);
   const int k = q[0].k, kg = k / q[0].gs;
@@ -235,8 +237,16 @@ void run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
     out[i] = outs[i].data_ptr(), ldo[i] = outs[i].stride(0);
   }
   const int64_t need = p_tf_qmm_set_scratch_bytes(count, n, sk);
+  if (need < 0 && optional) return false;
   if (need < 0) refuse("%s: bad shapes", who);
-  const at::Tensor scratch = scratch_of(x.get_device(), stream, need);
+  at::Tensor scratch;
+  try {
+    scratch = scratch_of(x.get_device(), stream, need);
+  } catch (const Refused&) {
+    if (!optional) throw;
+    PyErr_Clear();
+    return false;
+  }
   void* const area = scratch.data_ptr();
   const int64_t room = scratch.numel();
   const void* xp = x.data_ptr();
@@ -246,6 +256,7 @@ void run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
                               area, room, pdl, stream);
         }),
         who);
+  return true;
 }
 
 // Which of the two kernels for more than 16 rows (their bits are the same).  The tensor-memory kernel works on one block an
@@ -308,15 +319,14 @@ PyObject* matmul(PyObject* const* a) {
   const bool slices = sk > 1 && !reduce;
   at::Tensor out;
   if (a[5] != Py_None || !slices) out = out_of(a[5], m, q.n, f32 ? at::kFloat : at::kBFloat16, x, who);
-  if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices) {       // same bits, persistent launch
-    run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who);
+  // same bits, persistent launch (more slices than a cluster holds can also go through `part`, which needs no scratch area)
+  if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices && run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who, sk > CLUSTER_SLICES))
     return THPVariable_Wrap(out);
-  }
   const float* sums = sums_of(a[2], m, kg, who);
   if (truth(a[9]) && window_pays(m, q) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))
     return THPVariable_Wrap(out);
   at::Tensor part;
-  if (sk > 1 && (!reduce || sk > 8)) {
+  if (sk > 1 && (!reduce || sk > CLUSTER_SLICES)) {
     if (a[6] == Py_None) {
       part = empty({sk, m, q.n}, at::kFloat, x);
     } else {

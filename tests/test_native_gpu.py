@@ -52,3 +52,18 @@ def test_a_launch_holds_its_scratch_area(tmp_path):
         native.bind(str(_lib.LIB_PATH), _lib.ensure_device)
     assert taken and held not in taken
     assert torch.equal(qmm.matmul(x, q, sk=2), want)          # a new area, zeroed
+
+
+def test_a_capture_takes_many_slices_without_a_scratch_area():
+    """More than eight K slices can pass through memory that the graph owns, so such a call needs no area made before."""
+
+    q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 3)), 64)
+    x = synthetic.activations(4, 1024, 4).to(DEV)
+    want = qmm.matmul(x, q, sk=12)
+    torch.cuda.synchronize()
+    qmm.reset_scratch()
+    graph, out = torch.cuda.CUDAGraph(), torch.zeros_like(want)
+    with torch.cuda.graph(graph):
+        qmm.matmul(x, q, sk=12, out=out)
+    graph.replay()
+    assert torch.equal(out, want)
