@@ -157,6 +157,7 @@ SCRATCH_BYTES = 16 << 20          # one scratch area: room for a gate/up set of 
 SCRATCH_AREAS = 4                 # areas made on a device's first call: the calling stream's and three side streams'
 _set_scratch: dict = {}           # (device index, stream) -> the stream's scratch area
 _free_areas: dict = {}            # device index -> areas not yet handed to a stream
+_outgrown: list = []              # areas that were too small for a later call: graphs captured with them may still be replayed
 
 
 def _scratch_for(index: int, stream: int, need: int) -> torch.Tensor:
@@ -165,7 +166,8 @@ def _scratch_for(index: int, stream: int, need: int) -> torch.Tensor:
 
     Areas are made eagerly (four on a device's first call, more when a fifth stream shows up or a set needs more room)
     and only handed out during a stream capture: a graph must not own memory that later calls use, so a capture that
-    would need a new allocation is refused with a message saying which eager call to make first."""
+    would need a new allocation is refused with a message saying which eager call to make first.  An area that a stream
+    outgrows is kept for graphs; a new one is at least twice its size, so all of those are smaller than the last."""
 
     device, key = torch.device("cuda", index), (index, stream)
     buf = _set_scratch.get(key)
@@ -182,16 +184,22 @@ def _scratch_for(index: int, stream: int, need: int) -> torch.Tensor:
         raise RuntimeError("matmul_set: this call needs a new scratch area, which cannot be made while the stream is "
                            "capturing; run it once eagerly (any stream of this device) before the capture")
     else:
-        buf = torch.zeros((max(need, SCRATCH_BYTES),), dtype=torch.uint8, device=device)
+        size = max(need, SCRATCH_BYTES)
+        if buf is not None:
+            _outgrown.append(buf)
+            size = max(size, 2 * buf.numel())
+        buf = torch.zeros((size,), dtype=torch.uint8, device=device)
     _set_scratch[key] = buf
     return buf
 
 
 def reset_scratch() -> None:
-    """Forget every scratch area (after ``device_error`` reported a lost wait their counters may be non-zero)."""
+    """Forget every scratch area (after ``device_error`` reported a lost wait their counters may be non-zero).  Graphs
+    captured before must not be replayed after it: they use the areas of their time."""
 
     _set_scratch.clear()
     _free_areas.clear()
+    _outgrown.clear()
     _native().forget_scratch()
 
 

@@ -67,3 +67,30 @@ def test_a_capture_takes_many_slices_without_a_scratch_area():
         qmm.matmul(x, q, sk=12, out=out)
     graph.replay()
     assert torch.equal(out, want)
+
+
+def test_an_outgrown_area_stays_with_its_graphs():
+    """A graph captured with a stream's area is replayed after a larger set made the stream a new one: the first area's
+    memory must not have become another tensor's."""
+
+    qmm.reset_scratch()
+    q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 5)), 64)
+    wide = qmm.pack(*to_dev(*synthetic.raw_weight(128 * 150, 1024, 4, 64, 6)), 64)
+    x = synthetic.activations(4, 1024, 7).to(DEV)
+    want, out, graph, stream = qmm.matmul(x, q, sk=4), torch.zeros((4, 256), dtype=torch.bfloat16, device=DEV), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        qmm.matmul(x, q, sk=4, out=out)
+    key = (x.device.index, stream.cuda_stream)
+    held, size = qmm._set_scratch[key].data_ptr(), qmm._set_scratch[key].numel()
+    with torch.cuda.stream(stream):
+        qmm.matmul(x, wide, sk=16)                            # 150 blocks x 16 slices of 8 KB: more than an area holds
+    torch.cuda.synchronize()
+    others = [torch.full((size,), 255, dtype=torch.uint8, device=DEV) for _ in range(2 * qmm.SCRATCH_AREAS)]
+    with torch.cuda.stream(stream):
+        others += [torch.full((size,), 255, dtype=torch.uint8, device=DEV) for _ in range(2 * qmm.SCRATCH_AREAS)]
+    assert held not in [t.data_ptr() for t in others]
+    graph.replay()
+    assert torch.equal(out, want)
+    assert qmm._set_scratch[key].numel() >= 2 * size
+    qmm.reset_scratch()
