@@ -176,10 +176,14 @@ def _scratch_for(index: int, stream: int, need: int) -> torch.Tensor:
     capturing = torch.cuda.is_current_stream_capturing()
     free = _free_areas.setdefault(index, [])
     if not free and not capturing and not any(k[0] == index for k in _set_scratch):
-        free.extend(torch.zeros((SCRATCH_BYTES,), dtype=torch.uint8, device=device) for _ in range(SCRATCH_AREAS))
+        maker = torch.cuda.Stream(device=device)                # cleared for every stream, not only after this one's queue
+        with torch.cuda.stream(maker):
+            free.extend(torch.zeros((SCRATCH_BYTES,), dtype=torch.uint8, device=device) for _ in range(SCRATCH_AREAS))
+        maker.synchronize()
     fits = [i for i, area in enumerate(free) if area.numel() >= need]
     if buf is None and fits:
         buf = free.pop(fits[0])
+        buf.record_stream(torch.cuda.current_stream(device))    # freed, its memory waits for the work queued here
     elif capturing:
         raise RuntimeError("matmul_set: this call needs a new scratch area, which cannot be made while the stream is "
                            "capturing; run it once eagerly (any stream of this device) before the capture")

@@ -94,3 +94,22 @@ def test_an_outgrown_area_stays_with_its_graphs():
     assert torch.equal(out, want)
     assert qmm._set_scratch[key].numel() >= 2 * size
     qmm.reset_scratch()
+
+
+def test_an_area_is_clear_for_the_stream_that_gets_it():
+    """The first call makes the areas of later streams too; a stream that does not wait for that call's queue must find its
+    area zero.  Only the areas are looked at."""
+
+    qmm.reset_scratch()
+    torch.cuda.synchronize()
+    dirty = [torch.full((qmm.SCRATCH_BYTES,), 255, dtype=torch.uint8, device=DEV) for _ in range(2 * qmm.SCRATCH_AREAS)]
+    torch.cuda.synchronize()
+    assert dirty[0].any()                                      # (loads the kernel)
+    del dirty                                                  # their memory is what new areas get
+    index, first, second = torch.cuda.current_device(), torch.cuda.current_stream(), torch.cuda.Stream()
+    torch.cuda._sleep(200_000_000)                             # about a tenth of a second of queue on the first stream
+    qmm._scratch_for(index, first.cuda_stream, 1)
+    with torch.cuda.stream(second):
+        assert not qmm._scratch_for(index, second.cuda_stream, 1).any()
+    torch.cuda.synchronize()
+    qmm.reset_scratch()
