@@ -87,3 +87,21 @@ def test_graphs_own_their_counters_and_take_no_scratch_area():
                 graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(out, want) for out in outs) and _lib.device_error(x) == 0
+
+
+def test_a_capture_zeroes_its_counters_once():
+    """Each further call of a capture is one node, its kernel."""
+
+    from cuda.bindings import runtime
+
+    q, x = packed(4096, 4096, 64), synthetic.activations(48, 4096, 6).to(DEV)
+    out = qmm.matmul(x, q, sk=4)
+
+    def nodes(calls):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            for _ in range(calls):
+                qmm.matmul(x, q, sk=4, out=out)
+        return runtime.cudaGraphGetNodes(graph.raw_cuda_graph(), 0)[-1]
+
+    assert nodes(4) - nodes(1) == 3
