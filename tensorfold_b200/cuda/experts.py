@@ -204,20 +204,28 @@ def down(act: torch.Tensor, ex: Experts, plan: Plan, out: torch.Tensor, rows: in
     _grouped(act, 0, ex.down, ex.dims, ex.width, ex, plan, out, rows, 0, 0.0)
 
 
+def _fetchable(t: torch.Tensor, k: int) -> bool:
+    """bf16 rows of ``k`` that the prompt kernel reads where they are: unit stride, each on a 16-byte boundary."""
+
+    return (t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == k and t.stride(1) == 1 and t.stride(0) % 8 == 0
+            and t.data_ptr() % 16 == 0)
+
+
 def layer(x: torch.Tensor, ex: Experts, plan: Plan, act: torch.Tensor, out: torch.Tensor, rows: int) -> None:
     """``gate_up`` into ``act`` [R * slots, NI], then ``down`` into ``out`` [R * slots, D].  In the prefill form ``act`` holds the
-    activations in member order, so that ``down`` reads an expert's rows where they are; ``out`` is the same."""
+    activations in member order, so that ``down`` reads an expert's rows where they are; ``out`` is the same.  Buffers whose
+    rows cannot be read in place go through ``gate_up`` and ``down``, which copy or refuse them."""
 
-    if not plan.prefill or plan.experts > ex.count or x.dim() != 2 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+    pairs = rows * plan.slots
+    if pairs > plan.members.shape[0] or x.shape[0] < rows or act.shape[0] < pairs or out.shape[0] < pairs:
+        raise ValueError(f"experts: a plan, act and out of {pairs} pairs at least and {rows} rows of x are needed")
+    if not (plan.prefill and plan.experts <= ex.count and _fetchable(x, ex.dims) and _fetchable(act, ex.width)
+            and out.dtype in (torch.float32, torch.bfloat16) and out.dim() == 2 and out.shape[1] == ex.dims and out.stride(1) == 1):
         gate_up(x, ex, plan, act, rows)
         down(act, ex, plan, out, rows)
         return
-    if act.dtype != torch.bfloat16 or act.shape[1] != ex.width or x.dtype != torch.bfloat16 or x.shape[1] != ex.dims:
-        raise ValueError(f"experts: x must be (rows, {ex.dims}) and act (pairs, {ex.width}), both bf16")
-    if out.dtype not in (torch.float32, torch.bfloat16) or out.dim() != 2 or out.shape[1] != ex.dims or out.stride(1) != 1:
-        raise ValueError("experts: out must be (pairs, D) fp32 or bf16 with unit-stride rows")
     _prefill_format(ex)
-    lib, stream, pairs, rows_in = _lib.native(), _lib.stream_of(x), rows * plan.slots, _sorted(plan, ex, x)
+    lib, stream, rows_in = _lib.native(), _lib.stream_of(x), _sorted(plan, ex, x)
     items = min(max_items(pairs, plan.experts, plan.tile), plan.items.shape[0])
     lib.tf_moe_gather("experts (gather)", x, x.stride(0), plan.slots, plan.items, plan.counts, plan.members, pairs, ex.dims, rows_in, stream)
     lib.tf_moe_experts_sorted("experts (gate, up)", rows_in, ex.dims, ex.up, ex.up.stride(0), ex.count, (2 if ex.swiglu else 1) * ex.width,

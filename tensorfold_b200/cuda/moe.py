@@ -42,6 +42,7 @@ class MoEBuffers:
         self.wts = torch.empty((rows, slots), dtype=torch.float32, device=device)
         experts = cfg.num_experts + 1 if table_experts is None else table_experts
         self.plan = grouped.Plan(rows, slots, experts, device, prefill=prefill)
+        # [row, slot] in the decode form; the prefill form keeps its pairs in member order (by expert) instead
         self.act = torch.empty((rows, slots, cfg.moe_intermediate_size), dtype=torch.bfloat16, device=device)
         self.y = torch.empty((rows, slots, cfg.hidden_size), dtype=torch.bfloat16 if prefill else torch.float32,
                              device=device)

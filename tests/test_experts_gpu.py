@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import moe as omoe
-from tensorfold_b200 import synthetic
+from tensorfold_b200 import _lib, synthetic
 from tensorfold_b200.cuda import experts
 
 from gpu_util import DEV
@@ -253,4 +253,40 @@ def test_persistent_and_tiled_kernels_give_the_same_pairs(case):
     first = results[(0, 8)]
     for key, (act, y) in results.items():
         assert torch.equal(act, first[0]) and torch.equal(y, first[1]), key
+    assert _lib.device_error(x) == 0
+
+
+@pytest.mark.parametrize("prefill", [False, True])
+@pytest.mark.parametrize("case", CASES)
+def test_layer_equals_gate_up_then_down(case, prefill):
+    """Bit for bit, with ids that belong to no expert of the table (a rank's share) left alone, and with buffers whose rows
+    are strided, start off a 16-byte boundary or do not have unit stride."""
+
+    ex, _, _ = build(case, 31)
+    rows, y_dtype = 150, torch.bfloat16 if prefill else torch.float32
+    x = synthetic.activations(rows, ex.dims, 9, std=0.5).to(DEV)
+    for left_out in (False, True):
+        picks = picks_for(rows, case, 21)
+        if left_out:
+            picks = torch.where(picks % 3 == 1, -1, picks).to(torch.int32)
+        slots, pairs = picks.shape[1], picks.numel()
+        plan = experts.Plan(rows, slots, ex.count, DEV, prefill=prefill)
+        experts.route(picks, plan)
+        act, want = torch.zeros((pairs, ex.width), dtype=torch.bfloat16, device=DEV), torch.full((pairs, ex.dims), 7.0, dtype=y_dtype, device=DEV)
+        experts.gate_up(x, ex, plan, act, rows)
+        experts.down(act, ex, plan, want, rows)
+        assert bool((want[picks.reshape(-1) < 0] == 7.0).all())
+        wide = lambda pad: torch.zeros((pairs, ex.width + pad), dtype=torch.bfloat16, device=DEV)
+        for buf in (wide(0), wide(8)[:, :ex.width], wide(4)[:, :ex.width], wide(8)[:, 1:ex.width + 1]):
+            got = torch.full_like(want, 7.0)
+            experts.layer(x, ex, plan, buf, got, rows)
+            assert torch.equal(got, want), (left_out, buf.stride(), buf.data_ptr() % 16)
+        odd_out = torch.full((pairs, ex.dims + 3), 7.0, dtype=y_dtype, device=DEV)
+        experts.layer(x, ex, plan, wide(0), odd_out[:, :ex.dims], rows)
+        assert torch.equal(odd_out[:, :ex.dims], want) and bool((odd_out[:, ex.dims:] == 7.0).all())
+    bad = [dict(act=wide(ex.width)[:, ::2]), dict(act=wide(0).t()), dict(act=wide(0)[1:]), dict(out=want[1:]), dict(rows=rows + 1), dict(act=wide(0).float())]
+    for change in bad:
+        args = dict(act=wide(0), out=torch.zeros_like(want), rows=rows) | change
+        with pytest.raises(ValueError):
+            experts.layer(x, ex, plan, args["act"], args["out"], args["rows"])
     assert _lib.device_error(x) == 0
