@@ -733,8 +733,16 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const __nv_bfloat16* _
                                                           const int* __restrict__ counts, const int* __restrict__ members, int slots,
                                                           int pairs, int k, __nv_bfloat16* __restrict__ dst) {
   const int lane = threadIdx.x & 31, pos = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int n = counts[0];
-  if (n < 1 || pos >= min(pairs, items[3 * n - 2] + items[3 * n - 1])) return;        // (past the last item: not planned)
+  // members past the items hold no pair; a plan may list its items in any order
+  __shared__ int ends[8];
+  int end = 0;
+  for (int i = threadIdx.x, n = counts[0]; i < n; i += 256) end = max(end, items[3 * i + 1] + items[3 * i + 2]);
+  end = __reduce_max_sync(0xFFFFFFFFu, end);
+  if (lane == 0) ends[threadIdx.x >> 5] = end;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) end = max(end, ends[w]);
+  if (pos >= min(pairs, end)) return;
   const int pair = members[pos];
   if (pair < 0 || pair >= pairs) return;
   const int64_t row = slots > 0 ? pair / slots : pair;

@@ -290,3 +290,21 @@ def test_layer_equals_gate_up_then_down(case, prefill):
         with pytest.raises(ValueError):
             experts.layer(x, ex, plan, args["act"], args["out"], args["rows"])
     assert _lib.device_error(x) == 0
+
+
+def test_a_plan_lists_its_items_in_any_order():
+    case = CASES[1]
+    ex, _, _ = build(case, 41)
+    rows = 60
+    x = synthetic.activations(rows, ex.dims, 9, std=0.5).to(DEV)
+    act, y, plan = run(ex, x, picks_for(rows, case, 5), prefill=True)
+    n = int(plan.counts[0])
+    plan.items[:n] = plan.items[:n].flip(0)
+    plan.sorted.zero_()
+    again, y2 = torch.zeros_like(act), torch.zeros_like(y)
+    experts.gate_up(x, ex, plan, again, rows)
+    experts.down(again, ex, plan, y2, rows)
+    assert torch.equal(again, act) and torch.equal(y2, y)
+    plan.sorted.zero_(), y2.zero_()
+    experts.layer(x, ex, plan, again, y2, rows)
+    assert torch.equal(y2, y)
