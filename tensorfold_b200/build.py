@@ -14,6 +14,7 @@ import subprocess
 import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+from importlib.metadata import version
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -21,6 +22,7 @@ CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "libtensorfold_b200.so"
 NATIVE = HERE / "_native.so"
+NATIVE_FOR = OBJ / "native.for"       # what _native.so was compiled against
 BITS = (2, 3, 4, 5, 6, 8)
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--threads", "2"]
@@ -50,6 +52,18 @@ def _compile(unit) -> str:
     return obj.name
 
 
+def _native_for() -> str:
+    return f"torch {version('torch')}, {sys.implementation.cache_tag}"
+
+
+def _native_stale() -> bool:
+    """Sources or headers are newer, or torch or the interpreter is another one (their C++ interfaces have no stable ABI)."""
+
+    sources = CSRC / "native.cpp", HERE.parent / "include" / "tensorfold_b200.h"
+    return (not NATIVE.exists() or NATIVE.stat().st_mtime < max(s.stat().st_mtime for s in sources)
+            or not NATIVE_FOR.exists() or NATIVE_FOR.read_text() != _native_for())
+
+
 def _native() -> str:
     """Compiles the extension module against the torch that will load it."""
 
@@ -65,6 +79,7 @@ def _native() -> str:
     done = subprocess.run(cmd, capture_output=True, text=True)
     if done.returncode:
         raise RuntimeError(f"g++ failed for native.cpp:\n{done.stdout}\n{done.stderr}")
+    NATIVE_FOR.write_text(_native_for())
     return NATIVE.name
 
 
@@ -73,10 +88,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     heads = _newest_header()
     stale = [u for u in _units()
              if force or not u[1].exists() or u[1].stat().st_mtime < max(u[0].stat().st_mtime, heads)]
-    source = CSRC / "native.cpp"
-    native = force or not NATIVE.exists() or NATIVE.stat().st_mtime < max(
-        source.stat().st_mtime, (HERE.parent / "include" / "tensorfold_b200.h").stat().st_mtime)
-    jobs = ([_native] if native else []) + [lambda u=u: _compile(u) for u in stale]
+    jobs = ([_native] if force or _native_stale() else []) + [lambda u=u: _compile(u) for u in stale]
     if jobs:
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as pool:
             for name in pool.map(lambda job: job(), jobs):

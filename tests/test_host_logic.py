@@ -151,3 +151,17 @@ def test_decode_items_and_reduction_forms_follow_sizes_only():
                                      (8, 16 * 6144 + 8, 4, tp.PeerReducer.FLAGGED), (8, 2048 * 6144 + 8, 2, tp.PeerReducer.ALL)):
         red.world = world
         assert red.form(n, itemsize) == want, (world, n, itemsize)
+
+
+def test_the_extension_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    from tensorfold_b200 import build
+
+    made, made_for = tmp_path / "_native.so", tmp_path / "native.for"
+    monkeypatch.setattr(build, "NATIVE", made)
+    monkeypatch.setattr(build, "NATIVE_FOR", made_for)
+    assert build._native_stale()
+    made.touch()
+    made_for.write_text(build._native_for())
+    assert not build._native_stale()
+    monkeypatch.setattr(build, "version", lambda name: "0.0")
+    assert build._native_stale()
