@@ -260,13 +260,21 @@ bool run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
 }
 
 // Which of the two kernels for more than 16 rows (their bits are the same).  The tensor-memory kernel works on one block an
-// SM and its roles start one after another, about 4 us that the tiled kernel does not pay; that kernel in turn repeats its
-// conversion and its mma.sync for every 64 rows.  Measured at 4 bits, groups of 64, in us (tensor memory / tiled):
-// 17408 x 5120 36 / 31 at 17 rows, 37 / 33 at 32, 38 / 66 at 48, 142 / 254 at 256; 4096 x 4096 30 / 35 at 48; below the
-// line 1024 x 5120 22 / 18 at 64 and 128, above it 23 / 31 at 256; 256 x 512 12 / 8 at 17 to 256; 6 bits in groups of 128,
-// 2048 x 4096 21 / 17 at 64, 19 / 29 at 96.
-bool window_pays(int64_t m, const Weight& q) {
-  return m > 32 && (m + 63) / 64 * q.n * q.k >= (int64_t{1} << 24);
+// SM and its roles start one after another, about 4 us that the tiled kernel does not pay, for each launch of up to 256 rows;
+// that kernel in turn repeats its conversion and its mma.sync for every 64 rows, and makes the group sums again in every
+// column block unless they are given.  And one warp adds all slices of 32 columns while its block waits, so a slice has to be
+// worth it: the more slices there are, and the more affine steps (groups of 32) a weight costs.  Measured from graphs with
+// weights past L2, over 256 to 17408 columns, 512 to 16384 inputs, 33 to 600 rows and six formats: of 1445 calls of 2^24
+// products and more 4 are slower here than there, by 5% at most (242, by up to 2.2 times, without the slices' lines); with
+// sums given 49, near the lines, by 17% at most (347).  Times in us (tensor memory / tiled), 4 bits in groups of 64: 17408 x
+// 5120 in 4 slices 45 / 124 at 48 rows, 181 / 426 at 256; 1024 x 2048 15 / 13 at 48 and 53 / 50 at 600; 1536 x 4096 in 10
+// slices 38 / 50 at 256; 1024 x 8192 in 21 of 399 thousand weights 44 / 41 at 128; 2048 x 16384 in 37 141 / 108 at 128; in
+// groups of 32, 3072 x 5120 in 24 slices of 655 thousand 105 / 88 at 128, 4096 x 4096 in 18 of 932 thousand 37 / 44 at 33.
+bool window_pays(int64_t m, const Weight& q, int sk, bool sums) {
+  if (m <= 32 || sk > 32) return false;
+  const int64_t weights = static_cast<int64_t>(q.n) * q.k, work = (m + 63) / 64 * weights, launches = (m + 255) / 256;
+  const int64_t slice = (sk > 16 ? 720'000 : 600'000) * (q.gs == 32 ? 8 : 5) / 5;
+  return work >= (int64_t{1} << 24) && weights >= sk * slice && (launches == 1 || work >= launches * (sums ? 20'000'000 : 12'000'000));
 }
 
 // The counters of the tensor-memory kernel's slices: zero, and left zero by every launch.  An eager call uses its stream's
@@ -341,7 +349,7 @@ PyObject* matmul(PyObject* const* a) {
   if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices && run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who, sk > CLUSTER_SLICES))
     return THPVariable_Wrap(out);
   const float* sums = sums_of(a[2], m, kg, who);
-  if (truth(a[9]) && window_pays(m, q) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))
+  if (truth(a[9]) && window_pays(m, q, sk, sums != nullptr) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))
     return THPVariable_Wrap(out);
   at::Tensor part;
   if (sk > 1 && (!reduce || sk > CLUSTER_SLICES)) {

@@ -68,6 +68,16 @@ def test_matmul_gives_the_same_bits_on_both_sides_of_its_rule(monkeypatch, n, k,
     assert torch.equal(qmm.matmul(x, q), tiled(monkeypatch, x, q))
 
 
+@pytest.mark.parametrize("n,k,gs,sk", [(1536, 4096, 64, 10), (1536, 4096, 64, 11), (3072, 5120, 32, 16), (3072, 5120, 32, 17),
+                                       (2048, 8192, 64, 22), (2048, 8192, 64, 23), (4096, 8192, 64, 33)])
+@pytest.mark.parametrize("m", [192, 257])
+def test_matmul_gives_the_same_bits_on_both_sides_of_the_lines_for_slices(monkeypatch, n, k, gs, sk, m):
+    q, x = packed(n, k, gs), synthetic.activations(m, k, 7).to(DEV)
+    want = tiled(monkeypatch, x, q, sk=sk)
+    assert torch.equal(qmm.matmul(x, q, sk=sk), want)
+    assert torch.equal(qmm.matmul(x, q, qmm.group_sums(x, gs), sk=sk), want)
+
+
 def test_graphs_own_their_counters_and_take_no_scratch_area():
     """Graphs captured on one fresh stream replay side by side, and leave the sets' scratch areas to the sets."""
 
