@@ -266,7 +266,7 @@ bool run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
 // worth it: the more slices there are, and the more affine steps (groups of 32) a weight costs.  Measured from graphs with
 // weights past L2, over 256 to 17408 columns, 512 to 16384 inputs, 33 to 600 rows and six formats: of 1445 calls of 2^24
 // products and more 4 are slower here than there, by 5% at most (242, by up to 2.2 times, without the slices' lines); with
-// sums given 49, near the lines, by 17% at most (347).  Times in us (tensor memory / tiled), 4 bits in groups of 64: 17408 x
+// sums given 50, near the lines, by 17% at most (347).  Times in us (tensor memory / tiled), 4 bits in groups of 64: 17408 x
 // 5120 in 4 slices 45 / 124 at 48 rows, 181 / 426 at 256; 1024 x 2048 15 / 13 at 48 and 53 / 50 at 600; 1536 x 4096 in 10
 // slices 38 / 50 at 256; 1024 x 8192 in 21 of 399 thousand weights 44 / 41 at 128; 2048 x 16384 in 37 141 / 108 at 128; in
 // groups of 32, 3072 x 5120 in 24 slices of 655 thousand 105 / 88 at 128, 4096 x 4096 in 18 of 932 thousand 37 / 44 at 33.
@@ -331,6 +331,25 @@ bool run_window(const at::Tensor& x, const Weight& q, int sk, const float* sums,
   return true;
 }
 
+// Whether a call of up to 16 rows takes the persistent kernel: always up to eight slices.  With more the tiled kernel and a
+// second launch that adds the slices give the same bits and need no scratch.  A call alone is bound by its host path, so one
+// launch wins (1024 x 3456 at 16 rows 10.3 us against 12.3); in a graph the second launch costs a microsecond, and a persistent
+// kernel of few (column block, slice) units, whose blocks each start all of its roles, loses to it up to 16 slices: 4 bits in
+// groups of 64 at 9 rows, 1024 x 3456 (72 units) 8.6 / 7.7 us, 1024 x 5120 (104) 9.2 / 8.4, 2048 x 5120 (208) 10.4 / 10.7,
+// 1024 x 8192 in 21 slices 11.8 / 13.2.  With `pdl` it starts under the previous kernel's end and keeps up (256 x 5120 8.3 /
+// 8.4).  8-bit codes in groups of 128 over 8 rows, the most instructions a unit, are slower in it everywhere until the units
+// fill the machine: 16 rows, 512 x 12288 18.3 / 15.1, 4096 x 8192 (320 units) 30.1 / 27.2 (alone 30.8 / 28.8), 3072 x 16384
+// (504) 38.9 / 44.4.
+bool persistent_pays(int64_t m, const Weight& q, int sk, bool pdl, cudaStream_t stream) {
+  if (sk <= CLUSTER_SLICES) return true;
+  const int64_t units = (q.n + 127) / 128 * static_cast<int64_t>(sk);
+  if (q.bits == 8 && q.gs == 128 && m > 8 && units < 448) return false;
+  if (pdl || q.gs == 32 || sk > 16 || units >= 112) return true;
+  cudaStreamCaptureStatus status;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &status));
+  return status == cudaStreamCaptureStatusNone;
+}
+
 // matmul(x, q, xs, sk, f32, out, part, reduce, pdl, stream)
 PyObject* matmul(PyObject* const* a) {
   const char* who = "matmul";
@@ -345,8 +364,8 @@ PyObject* matmul(PyObject* const* a) {
   const bool slices = sk > 1 && !reduce;
   at::Tensor out;
   if (a[5] != Py_None || !slices) out = out_of(a[5], m, q.n, f32 ? at::kFloat : at::kBFloat16, x, who);
-  // same bits, persistent launch (more slices than a cluster holds can also go through `part`, which needs no scratch area)
-  if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices && run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who, sk > CLUSTER_SLICES))
+  if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices && persistent_pays(m, q, sk, pdl, stream) &&
+      run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who, sk > CLUSTER_SLICES))
     return THPVariable_Wrap(out);
   const float* sums = sums_of(a[2], m, kg, who);
   if (truth(a[9]) && window_pays(m, q, sk, sums != nullptr) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))

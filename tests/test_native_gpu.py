@@ -54,7 +54,8 @@ def test_a_launch_holds_its_scratch_area(tmp_path):
     assert torch.equal(qmm.matmul(x, q, sk=2), want)          # a new area, zeroed
 
 
-def test_a_capture_takes_many_slices_without_a_scratch_area():
+@pytest.mark.parametrize("pdl", [False, True])
+def test_a_capture_takes_many_slices_without_a_scratch_area(pdl):
     """More than eight K slices can pass through memory that the graph owns, so such a call needs no area made before."""
 
     q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 3)), 64)
@@ -64,7 +65,7 @@ def test_a_capture_takes_many_slices_without_a_scratch_area():
     qmm.reset_scratch()
     graph, out = torch.cuda.CUDAGraph(), torch.zeros_like(want)
     with torch.cuda.graph(graph):
-        qmm.matmul(x, q, sk=12, out=out)
+        qmm.matmul(x, q, sk=12, out=out, pdl=pdl)
     graph.replay()
     assert torch.equal(out, want)
 

@@ -157,3 +157,24 @@ def test_c_abi_refuses_bad_sets():
     assert call(nproj=5) < 0
     torch.cuda.synchronize()
     assert _lib.device_error(x) == 0
+
+
+@pytest.mark.parametrize("bits,gs,n,sk", [(4, 64, 256, 9), (4, 64, 384, 16), (4, 64, 384, 17), (4, 64, 896, 16), (6, 128, 128, 12), (3, 32, 256, 9),
+                                          (8, 128, 128, 9), (8, 128, 2048, 28), (8, 128, 2040, 27)])
+def test_calls_of_many_slices_keep_their_bits_on_every_route(bits, gs, n, sk):
+    """More than eight slices: the persistent kernel or the tiled one with a second launch, eager or captured."""
+
+    q, x = packed(n, 40 * gs, gs, 3 * n + sk, bits), synthetic.activations(16, 40 * gs, 8).to(DEV)
+    want = tiled_kernel(x, q, sk=sk)
+    for m in (1, 8, 9, 16):
+        out = torch.zeros((2, m, n), dtype=torch.bfloat16, device=DEV)
+        assert torch.equal(qmm.matmul(x[:m], q, sk=sk), want[:m])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for pdl in (False, True):
+                qmm.matmul(x[:m], q, sk=sk, out=out[int(pdl)], pdl=pdl)
+        graph.replay()
+        assert torch.equal(out[0], want[:m]) and torch.equal(out[1], want[:m])
+    assert _lib.device_error(x) == 0
+    del graph
+    qmm.reset_scratch()                                       # (the capture stream took one of the areas)
