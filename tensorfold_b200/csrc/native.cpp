@@ -336,15 +336,16 @@ bool run_window(const at::Tensor& x, const Weight& q, int sk, const float* sums,
 // launch wins (1024 x 3456 at 16 rows 10.3 us against 12.3); in a graph the second launch costs a microsecond, and a persistent
 // kernel of few (column block, slice) units, whose blocks each start all of its roles, loses to it up to 16 slices: 4 bits in
 // groups of 64 at 9 rows, 1024 x 3456 (72 units) 8.6 / 7.7 us, 1024 x 5120 (104) 9.2 / 8.4, 2048 x 5120 (208) 10.4 / 10.7,
-// 1024 x 8192 in 21 slices 11.8 / 13.2.  With `pdl` it starts under the previous kernel's end and keeps up (256 x 5120 8.3 /
-// 8.4).  8-bit codes in groups of 128 over 8 rows, the most instructions a unit, are slower in it everywhere until the units
-// fill the machine: 16 rows, 512 x 12288 18.3 / 15.1, 4096 x 8192 (320 units) 30.1 / 27.2 (alone 30.8 / 28.8), 3072 x 16384
-// (504) 38.9 / 44.4.
+// 1024 x 8192 in 21 slices 11.8 / 13.2.  With `pdl` both kernels start under the previous one's end, and the few units of very
+// small projections as well in the one as in the other: 256 x 5120 (26) 8.3 / 8.4, 1024 x 5120 (104) 9.2 / 7.9, 1536 x 5120
+// (156) 10.0 / 9.3, 2048 x 5120 (208) 10.1 / 10.1.  8-bit codes in groups of 128 over 8 rows, the most instructions a unit, are
+// slower in it everywhere until the units fill the machine: 16 rows, 512 x 12288 18.3 / 15.1, 4096 x 8192 (320 units) 30.1 /
+// 27.2 (alone 30.8 / 28.8), 3072 x 16384 (504) 38.9 / 44.4.
 bool persistent_pays(int64_t m, const Weight& q, int sk, bool pdl, cudaStream_t stream) {
   if (sk <= CLUSTER_SLICES) return true;
   const int64_t units = (q.n + 127) / 128 * static_cast<int64_t>(sk);
   if (q.bits == 8 && q.gs == 128 && m > 8 && units < 448) return false;
-  if (pdl || q.gs == 32 || sk > 16 || units >= 112) return true;
+  if (q.gs == 32 || sk > 16 || (pdl ? units < 48 || units >= 200 : units >= 112)) return true;
   cudaStreamCaptureStatus status;
   C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &status));
   return status == cudaStreamCaptureStatusNone;
