@@ -272,7 +272,8 @@ def test_layer_equals_gate_up_then_down(case, prefill):
         slots, pairs = picks.shape[1], picks.numel()
         plan = experts.Plan(rows, slots, ex.count, DEV, prefill=prefill)
         experts.route(picks, plan)
-        act, want = torch.zeros((pairs, ex.width), dtype=torch.bfloat16, device=DEV), torch.full((pairs, ex.dims), 7.0, dtype=y_dtype, device=DEV)
+        act = torch.zeros((pairs, ex.width), dtype=torch.bfloat16, device=DEV)
+        want = torch.full((pairs, ex.dims), 7.0, dtype=y_dtype, device=DEV)
         experts.gate_up(x, ex, plan, act, rows)
         experts.down(act, ex, plan, want, rows)
         assert bool((want[picks.reshape(-1) < 0] == 7.0).all())
@@ -284,7 +285,8 @@ def test_layer_equals_gate_up_then_down(case, prefill):
         odd_out = torch.full((pairs, ex.dims + 3), 7.0, dtype=y_dtype, device=DEV)
         experts.layer(x, ex, plan, wide(0), odd_out[:, :ex.dims], rows)
         assert torch.equal(odd_out[:, :ex.dims], want) and bool((odd_out[:, ex.dims:] == 7.0).all())
-    bad = [dict(act=wide(ex.width)[:, ::2]), dict(act=wide(0).t()), dict(act=wide(0)[1:]), dict(out=want[1:]), dict(rows=rows + 1), dict(act=wide(0).float())]
+    bad = [dict(act=wide(ex.width)[:, ::2]), dict(act=wide(0).t()), dict(act=wide(0)[1:]), dict(act=wide(0).float()),
+           dict(out=want[1:]), dict(rows=rows + 1)]
     for change in bad:
         args = dict(act=wide(0), out=torch.zeros_like(want), rows=rows) | change
         with pytest.raises(ValueError):

@@ -78,7 +78,8 @@ def test_an_outgrown_area_stays_with_its_graphs():
     q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 5)), 64)
     wide = qmm.pack(*to_dev(*synthetic.raw_weight(128 * 150, 1024, 4, 64, 6)), 64)
     x = synthetic.activations(4, 1024, 7).to(DEV)
-    want, out, graph, stream = qmm.matmul(x, q, sk=4), torch.zeros((4, 256), dtype=torch.bfloat16, device=DEV), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    want, graph, stream = qmm.matmul(x, q, sk=4), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    out = torch.zeros_like(want)
     torch.cuda.synchronize()
     with torch.cuda.graph(graph, stream=stream):
         qmm.matmul(x, q, sk=4, out=out)

@@ -159,8 +159,9 @@ def test_c_abi_refuses_bad_sets():
     assert _lib.device_error(x) == 0
 
 
-@pytest.mark.parametrize("bits,gs,n,sk", [(4, 64, 256, 9), (4, 64, 384, 15), (4, 64, 384, 16), (4, 64, 384, 17), (4, 64, 896, 16), (4, 64, 1600, 16), (6, 128, 128, 12), (3, 32, 256, 9),
-                                          (8, 128, 128, 9), (8, 128, 2048, 28), (8, 128, 2040, 27)])
+@pytest.mark.parametrize("bits,gs,n,sk", [(4, 64, 256, 9), (4, 64, 384, 15), (4, 64, 384, 16), (4, 64, 384, 17), (4, 64, 896, 16),
+                                          (4, 64, 1600, 16), (6, 128, 128, 12), (3, 32, 256, 9), (8, 128, 128, 9),
+                                          (8, 128, 2048, 28), (8, 128, 2040, 27)])
 def test_calls_of_many_slices_keep_their_bits_on_every_route(bits, gs, n, sk):
     """More than eight slices: the persistent kernel or the tiled one with a second launch, eager or captured."""
 

@@ -62,6 +62,78 @@ def test_every_format(monkeypatch, bits, gs):
         assert torch.equal(window(x[:m], q, sk=sk, f32=True), tiled(monkeypatch, x[:m], q, sk=sk, f32=True))
 
 
+def hard(kind, m, k):
+    """Rows whose 16-input steps a differently aligned or truncating adder would round to other bits."""
+
+    g = torch.Generator().manual_seed(len(kind) * 1000 + k)
+    x = torch.randn((m, k), generator=g)
+    powers = lambda lo, hi: torch.exp2(torch.randint(lo, hi, (m, k), generator=g).float())
+    if kind == "spread":                                     # exponents over 60 and over 200 binades
+        x[: m // 2] *= powers(-30, 31)[: m // 2]
+        x[m // 2:] *= powers(-100, 101)[m // 2:]
+    elif kind == "cancelling":                               # v, -v beside much smaller terms, next to each other and apart
+        x = (x * powers(-8, 9)).bfloat16().float()
+        big = (torch.randn((m, k // 2), generator=g) * 2 ** 20).bfloat16().float() * (torch.rand((m, k // 2), generator=g) < 0.3)
+        x[:, 0::2] = torch.where(big != 0, big, x[:, 0::2])
+        x[:, 1::2] = torch.where(big != 0, -big, x[:, 1::2])
+        x[1::2] = x[1::2, torch.randperm(k, generator=g)]
+    elif kind == "subnormal":
+        x[: m // 2] *= 2.0 ** -128
+        x[m // 2:] *= powers(-133, -100)[m // 2:]
+    elif kind == "large":                                    # sums past the largest finite value
+        x *= 2.0 ** 118
+    elif kind == "zeros":
+        x = torch.where(torch.rand((m, k), generator=g) < 0.5, -0.0, 0.0)
+        x[: m // 2] = -0.0
+    else:                                                    # infinities and NaN here and there
+        r = torch.rand((m, k), generator=g)
+        x[r < 0.0005], x[(r > 0.0005) & (r < 0.001)], x[r > 0.9997] = float("inf"), -float("inf"), float("nan")
+    return x.to(torch.bfloat16).to(DEV)
+
+
+@pytest.mark.parametrize("kind", ["spread", "cancelling", "subnormal", "large", "zeros", "infinite"])
+@pytest.mark.parametrize("bits,gs", [(2, 128), (3, 32), (4, 32), (4, 64), (4, 128), (5, 64), (6, 128)])
+def test_sums_that_are_hard_to_round_carry_the_same_bits(monkeypatch, kind, bits, gs):
+    """Rows keep their bits between up to 16 (persistent kernel), 32 and more rows, which run on mma.sync and on tcgen05.mma:
+    their accumulation steps must round alike for every input.  A NaN is a NaN, whatever its bits."""
+
+    q, x = packed(328, gs * 13, gs, bits), hard(kind, 64, gs * 13)
+    bits_of = lambda t: t.masked_fill(t.isnan(), 0).view(torch.int32)
+    same = lambda a, b: torch.equal(a.isnan(), b.isnan()) and torch.equal(bits_of(a), bits_of(b))
+    for m, sk in ((40, 1), (64, 3)):
+        want = tiled(monkeypatch, x[:m], q, sk=sk, f32=True)
+        assert same(window(x[:m], q, sk=sk, f32=True), want)
+        assert same(qmm.matmul(x[:16], q, sk=sk, f32=True), want[:16])
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_chain_of_calls_with_pdl(monkeypatch, captured):
+    """Each call reads the rows the one before it writes, starts before that one has ended, and shares its counters."""
+
+    n = 4096
+    qs, x = [packed(n, n, 64), packed(n, n, 64, 3)], synthetic.activations(48, n, 6, std=2 ** -10).to(DEV)
+    outs = [torch.zeros((48, n), dtype=torch.bfloat16, device=DEV) for _ in range(6)]
+
+    def chain(matmul, outs, **kw):
+        for i, out in enumerate(outs):
+            matmul(outs[i - 1] if i else x, qs[i % 2], sk=4, out=out, **kw)
+
+    want = [torch.zeros_like(out) for out in outs]
+    chain(lambda *a, **kw: tiled(monkeypatch, *a, **kw), want)
+    chain(qmm.matmul, outs, pdl=True)
+    if captured:
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            chain(qmm.matmul, outs, pdl=True)
+        for _ in range(3):
+            for out in outs:
+                out.zero_()
+            graph.replay()
+    assert all(out.isfinite().all() and torch.equal(out, ref) for out, ref in zip(outs, want)) and outs[-1].any()
+    assert _lib.device_error(x) == 0
+
+
 @pytest.mark.parametrize("n,k,m", [(4096, 4096, 32), (4096, 4096, 33), (4095, 4096, 64), (1024, 5120, 192), (1024, 5120, 256)])
 def test_matmul_gives_the_same_bits_on_both_sides_of_its_rule(monkeypatch, n, k, m):
     q, x = packed(n, k, 64), synthetic.activations(m, k + 8, 7).to(DEV)[:, :k]
