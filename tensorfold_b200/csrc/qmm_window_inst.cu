@@ -27,8 +27,14 @@ cudaError_t launch(const CUtensorMap& tmx, const WindowParams& p, int grid, cuda
 
 template <int GS, int ROWS>
 cudaError_t configure() {
-  return cudaFuncSetAttribute(qmm_window_kernel<TF_BITS, GS, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              WindowGeo<TF_BITS, GS, ROWS>::SMEM);
+  using Geo = WindowGeo<TF_BITS, GS, ROWS>;
+  // The roles' shares (setmaxnreg) add up to 96 registers a thread.  A kernel compiled to fewer would wait for ever for its
+  // epilogue warps' share, so it must not be launched.
+  cudaFuncAttributes compiled;
+  cudaError_t e = cudaFuncGetAttributes(&compiled, qmm_window_kernel<TF_BITS, GS, ROWS>);
+  if (e == cudaSuccess && compiled.numRegs < 96) e = cudaErrorLaunchOutOfResources;
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(qmm_window_kernel<TF_BITS, GS, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM);
 }
 
 }  // namespace
