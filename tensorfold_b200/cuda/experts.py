@@ -216,10 +216,14 @@ def layer(x: torch.Tensor, ex: Experts, plan: Plan, act: torch.Tensor, out: torc
     activations in member order, so that ``down`` reads an expert's rows where they are; ``out`` is the same.  Buffers whose
     rows cannot be read in place go through ``gate_up`` and ``down``, which copy or refuse them."""
 
+    if not plan.prefill:
+        gate_up(x, ex, plan, act, rows)
+        down(act, ex, plan, out, rows)
+        return
     pairs = rows * plan.slots
     if pairs > plan.members.shape[0] or x.shape[0] < rows or act.shape[0] < pairs or out.shape[0] < pairs:
         raise ValueError(f"experts: a plan, act and out of {pairs} pairs at least and {rows} rows of x are needed")
-    if not (plan.prefill and plan.experts <= ex.count and _fetchable(x, ex.dims) and _fetchable(act, ex.width)
+    if not (plan.experts <= ex.count and _fetchable(x, ex.dims) and _fetchable(act, ex.width)
             and out.dtype in (torch.float32, torch.bfloat16) and out.dim() == 2 and out.shape[1] == ex.dims and out.stride(1) == 1):
         gate_up(x, ex, plan, act, rows)
         down(act, ex, plan, out, rows)
