@@ -99,7 +99,9 @@ int tf_group_sums(const void* x, int64_t ldx, int m, int k, int gs, float* xs, v
  *            chip; more pass through part and a second kernel), else may be NULL
  *   reduce   1: out receives the sum of the slices; 0: the slices stay in part (out untouched)
  *   pdl      1: launch with programmatic stream serialisation, so this call's weight prefetch overlaps the tail of the
- *            previous kernel in the stream (it still waits for that kernel before reading x or writing out)
+ *            previous kernel in the stream (it still waits for that kernel before reading x or writing out).  So with
+ *            pdl = 1, here and in every entry that has the argument, the weights must be settled: no kernel still in
+ *            flight writes them.  tf_qmm_prefill and its forms have no such precondition
  * Replaces the pybind function qmm(x, xs, w, scales, biases, out, part, n, sk, gs, bm, f32, reduce) of
  * cuda/kernels/qmm.cpp:14-44 and, for bits != 4, the Triton launch of cuda/kernels/affine.py:53-68. */
 int tf_qmm(const void* x, int64_t ldx, int m, const float* xs, const void* tiled, int64_t sb_stride, int n, int k,
@@ -189,9 +191,10 @@ int tf_moe_experts_prefill(const void* x, int64_t ldx, int slots, const void* ti
                            int k, int gs, const int* items, const int* counts, const int* members, int pairs, int max_items,
                            void* sorted, void* out, int64_t ldo, int out_f32, int epi, float limit, void* stream);
 /* The two halves of tf_moe_experts_prefill, for a layer that keeps its activations in member order between its two
- * projections.  tf_moe_gather: sorted[pos] = row members[pos] / slots of x (members[pos] with slots 0) for every planned
- * pair.  tf_moe_experts_sorted: `sorted` holds the rows in member order, ldx elements apart; out row members[pos], or with
- * members NULL row pos, which is the next projection's input as it stands. */
+ * projections.  tf_moe_gather: sorted[pos] = row members[pos] / slots of x (members[pos] with slots 0) for every position
+ * up to the largest end of the plan's items, which may be listed in any order.  tf_moe_experts_sorted: `sorted` holds
+ * the rows in member order, ldx elements apart; out row members[pos], or with members NULL row pos, which is the next
+ * projection's input as it stands. */
 int tf_moe_gather(const void* x, int64_t ldx, int slots, const int* items, const int* counts, const int* members, int pairs, int k,
                   void* sorted, void* stream);
 int tf_moe_experts_sorted(const void* sorted, int64_t ldx, const void* tiled, int64_t expert_stride, int experts, int n, int k, int gs,
@@ -278,7 +281,7 @@ int tf_swiglu(const void* gate, const void* up, int rows, int n, void* out, floa
 
 /* Prefill matmul on tcgen05 / tensor memory: every weight rounded once to bf16, w = bf16(fma(q, s, b)), then one fp32
  * accumulation chain over K; any chunking of the rows gives the same bits (not the bits of tf_qmm).  4-bit weights,
- * groups of 32 or 64, k % 64 == 0.  x: [m, k] bf16, 16-byte aligned rows (ldx % 8 == 0); out: [m, n] bf16 or fp32.
+ * groups of 32 or 64, k a multiple of the group.  x: [m, k] bf16, 16-byte aligned rows (ldx % 8 == 0); out: [m, n] bf16 or fp32.
  * Replaces the pybind function qmm_prefill(x, w, scales, biases, out, n, gs, f32, tile) of cuda/kernels/qmm.cpp:47-66
  * (cuda/kernels/qmm_prefill.cu:36-191). */
 int tf_qmm_prefill(const void* x, int64_t ldx, int m, const void* tiled, int64_t sb_stride, int n, int k, int gs, void* out,

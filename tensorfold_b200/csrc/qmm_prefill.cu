@@ -23,9 +23,10 @@
 // issues the MMAs, warp 2 loads packed units, warps 4-19 are two groups of eight conversion warps that take alternate
 // stages, warps 20-27 drain the finished accumulator.  Barriers the MMA warp waits on live in the first block; the second
 // block's copies and conversion warps signal them across the pair.
-// Measured, one projection by CUDA events (in brackets one block a tile with A in shared memory): 2048 rows, 17408 x 5120
-// 246 us = 1484 TFLOP/s (335), 5120 x 17408 242 us (402), 1024 x 5120 21 us (53); 391 rows, 17408 x 5120 54 us (90); 64 rows,
-// 6144 x 5120 17 us (45).  cuBLAS does 8192^3 in bf16 at 1672 TFLOP/s here, 1424 over seconds: both are bound by power.
+// Measured, one projection by CUDA events from a graph (in brackets in us: one block a tile with A in shared memory): 2048 rows,
+// 17408 x 5120 240 us = 1522 TFLOP/s (335), 5120 x 17408 238 us (402), 1024 x 5120 20 us (53); 391 rows, 17408 x 5120 54 us
+// (90); 64 rows, 6144 x 5120 17 us (45).  The tensor pipe is active in 92 % of the cycles of the first of these.  cuBLAS does
+// 8192^3 in bf16 at 1696 TFLOP/s here, 1427 over seconds: both are bound by power.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const __grid_con
     // ------------------------------------------------------------------ MMA issue (one thread of the first block)
     if (half == 0) {
       // The tensor pipe's queue is short, so this warp must stay ahead of it: one barrier a stage, eight MMAs a barrier,
-      // and addresses that are the same in every lane (elect.sync lets the compiler keep them in uniform registers:
-      // 32 cycles an MMA of 64 rows against 78 for a loop behind `lane == 0`).
+      // and addresses that are the same in every lane (elect.sync lets the compiler keep them in uniform registers, which it
+      // does not do in a loop behind `lane == 0`).
       const uint32_t full32 = smem_addr(full), empty32 = smem_addr(empty), acc_full32 = smem_addr(acc_full);
       const uint64_t bd0 = umma_desc(smem_addr(smem));
       const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);

@@ -18,11 +18,14 @@
 // Row tiles come first in the item order, so the tiles that share weights run at the same time and find them in L2.  Slices
 // meet in global memory as in qmm_stream.cuh: the warp that counts itself in last adds them in slice order.
 // Blocks never wait for one another.  `count` is zero before and after every launch.
-// What bounds it now is instruction issue and latency inside a block, not memory: a pair of groups (one a super-block) takes
-// about 1000 cycles, most of them the epilogue's, against 260 of MMAs; code is kept short (the slice sum is a loop over sixteen
-// rows), since a first pass over it is fetched from L2.
-// Measured (48 rows, 4 bits, groups of 64; the tiled kernel in brackets): 17408 x 5120 37.7 us (65.6), 5120 x 17408 52 (80),
-// 6144 x 5120 33 (42), 5120 x 6144 36 (48); 256 rows, 17408 x 5120 142 us (254).
+// What bounds it now is the chain inside a block, not memory and not the tensor pipe (12 % of active cycles at 48 rows): a pair
+// of groups (one a super-block) takes about 1200 cycles, at 16 rows nearly as many as at 48 (17408 x 5120 in one slice, 80 pairs
+// one after another: 53.2 us at 16 rows, 54.6 at 48, 62.0 at 64), so it is waits and round trips through tensor memory rather
+// than the epilogue's arithmetic.  Code is kept short (the slice sum is a loop over sixteen rows), since a first pass over it is
+// fetched from L2.
+// Measured from graphs, weights past L2, sums given (4 bits, groups of 64; the tiled kernel in brackets): 48 rows, 17408 x 5120
+// 37.3 us (66.0), 5120 x 17408 50.0 (77.7), 6144 x 5120 31.9 (38.9), 5120 x 6144 34.2 (44.6); 256 rows, 17408 x 5120 140 us
+// (254), 5120 x 17408 227 (305).
 #pragma once
 
 #include "qmm_tiled.cuh"

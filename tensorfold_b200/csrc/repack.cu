@@ -7,8 +7,9 @@
 // whole lanes (pack) or whole rows (unpack), so positions are compile-time constants, codes move in pairs (inputs 2 i,
 // 2 i + 1 are neighbours in the stored row and the two halves of one lane word), and 4-bit codes, the common width, move
 // four bytes at a time with byte permutes.
-// Measured, 17408 x 5120 (pack / unpack): 4 bits 33 / 23 us (3.0 / 4.4 TB/s), 8 bits 57 / 50 us, 3 bits 50 / 41 us.  One
-// thread an output word, gathering its codes from global memory, took 252 / 289 us at 4 bits.
+// Measured from graphs, 17408 x 5120 in groups of 64 (pack / unpack): 4 bits 29 / 22 us (3.5 / 4.6 TB/s), 8 bits 51 / 49 us (3.7 /
+// 3.9), 3 bits 45 / 39 us (1.7 / 2.0), 2 bits 21 / 22, 5 bits 63 / 50, 6 bits 54 / 54.  One thread an output word, gathering its
+// codes from global memory, took 252 / 289 us at 4 bits.
 #include <algorithm>
 #include <type_traits>
 

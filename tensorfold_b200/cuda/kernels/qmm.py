@@ -147,7 +147,7 @@ def matmul(x: torch.Tensor, q: Q4, xs: torch.Tensor | None = None, *, sk: int | 
     """x @ q.T as (M, n) bf16, or unrounded fp32 with ``f32``; ``reduce=False`` returns K slices to add in order.
 
     ``pdl`` (not in the reference) launches with programmatic stream serialisation so the weight prefetch of this call
-    overlaps the end of the previous kernel in the stream."""
+    overlaps the end of the previous kernel in the stream: the weights must not be what a kernel still in flight writes."""
 
     return _native().matmul(x, q, xs, sk, f32, out, part, reduce, pdl, STREAM)
 
