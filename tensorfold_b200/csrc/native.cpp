@@ -162,9 +162,16 @@ at::Tensor rows_of(const at::Tensor& x, int k, const char* who) {
   return x;
 }
 
-const float* sums_of(PyObject* xs, int64_t m, int64_t kg, const char* who) {
+// Kernels reach any CUDA memory and pinned host memory, nothing else.
+void reachable(const at::Tensor& t, const char* what, const char* who) {
+  if (t.is_cpu() && !t.is_pinned()) refuse("%s: %s lives in host memory that the device cannot reach", who, what);
+}
+
+const float* sums_of(PyObject* xs, const at::Tensor& x, int64_t kg, const char* who) {
   if (xs == Py_None) return nullptr;
   const at::Tensor& t = tensor(xs, who);
+  const int64_t m = x.size(0);
+  reachable(t, "xs", who);
   if (t.scalar_type() != at::kFloat || t.dim() != 2 || t.size(0) != m || t.size(1) != kg || !t.is_contiguous())
     refuse("%s: xs must be contiguous (%lld, %lld) fp32", who, static_cast<long long>(m), static_cast<long long>(kg));
   return t.data_ptr<float>();
@@ -176,6 +183,7 @@ at::Tensor out_of(PyObject* out, int64_t m, int64_t n, at::ScalarType type, cons
   const at::Tensor& t = tensor(out, who);
   if (t.dim() != 2 || t.size(0) != m || t.size(1) != n || t.scalar_type() != type || t.stride(1) != 1)
     refuse("%s: out must be (M, n) of the requested dtype with unit-stride rows", who);
+  reachable(t, "out", who);
   return t;
 }
 
@@ -225,7 +233,7 @@ bool run_set(const at::Tensor& x, const Weight* q, const int* sk, int count, PyO
   const cudaStream_t stream = stream_of(x);
   const int64_t m = x.size(0);
   const int k = q[0].k, kg = k / q[0].gs;
-  const float* sums = sums_of(xs, m, kg, who);
+  const float* sums = sums_of(xs, x, kg, who);
   const void* tiled[SET_MAX];
   void* out[SET_MAX];
   int64_t stride[SET_MAX], ldo[SET_MAX];
@@ -368,7 +376,7 @@ PyObject* matmul(PyObject* const* a) {
   if (truth(a[9]) && m <= SET_ROWS && a[6] == Py_None && !slices && persistent_pays(m, q, sk, pdl, stream) &&
       run_set(x, &q, &sk, 1, a[2], f32, &out, pdl, who, sk > CLUSTER_SLICES))
     return THPVariable_Wrap(out);
-  const float* sums = sums_of(a[2], m, kg, who);
+  const float* sums = sums_of(a[2], x, kg, who);
   if (truth(a[9]) && window_pays(m, q, sk, sums != nullptr) && a[6] == Py_None && !slices && run_window(x, q, sk, sums, f32, out, pdl, stream, who))
     return THPVariable_Wrap(out);
   at::Tensor part;
@@ -379,6 +387,7 @@ PyObject* matmul(PyObject* const* a) {
       part = tensor(a[6], who);
       if (part.scalar_type() != at::kFloat || !part.is_contiguous() || part.numel() < sk * m * q.n)
         refuse("matmul: part must hold (SK, M, n) fp32");
+      reachable(part, "part", who);
     }
   }
   check(unlocked([&] {
@@ -432,6 +441,7 @@ PyObject* prefill_matmul(PyObject* const* a) {
   const Weight q(a[1]);
   const at::Tensor x = rows_of(tensor(a[0], who), q.k, who);
   const cudaStream_t stream = stream_of(x);
+  reachable(q.units, "the weight", who);
   const bool f32 = truth(a[2]);
   const at::Tensor out = out_of(a[3], x.size(0), q.n, f32 ? at::kFloat : at::kBFloat16, x, who);
   check(unlocked([&] {
@@ -448,6 +458,7 @@ PyObject* matmul_act(PyObject* const* a) {
   const Weight q(a[1]);
   const at::Tensor x = rows_of(tensor(a[0], who), q.k, who);
   const cudaStream_t stream = stream_of(x);
+  reachable(q.units, "the weight", who);
   const bool swiglu = truth(a[2]), pdl = truth(a[5]), prefill = truth(a[6]) && q.bits == 4 && (q.gs == 32 || q.gs == 64);
   const float limit = static_cast<float>(number(a[3]));
   const int epi = swiglu ? 2 : 1, m = static_cast<int>(x.size(0));

@@ -115,3 +115,23 @@ def test_an_area_is_clear_for_the_stream_that_gets_it():
         assert not qmm._scratch_for(index, second.cuda_stream, 1).any()
     torch.cuda.synchronize()
     qmm.reset_scratch()
+
+
+def test_host_memory_is_refused_unless_it_is_pinned():
+    """An address that the device cannot reach must not get to a kernel, whichever operand brings it."""
+
+    q = qmm.pack(*to_dev(*synthetic.raw_weight(256, 1024, 4, 64, 8)), 64)
+    host = qmm.Q4(q.weight.cpu(), None, None, q.n, q.k, q.gs)
+    for m in (4, 24):
+        x, out = synthetic.activations(m, 1024, 9).to(DEV), torch.empty((m, 256), dtype=torch.bfloat16)
+        calls = [lambda: qmm.matmul(x, host), lambda: qmm.prefill_matmul(x, host), lambda: qmm.matmul_act(x, host, act="relu2"),
+                 lambda: qmm.matmul_act(x, host, act="relu2", prefill=True), lambda: qmm.matmul(x, q, out=out),
+                 lambda: qmm.prefill_matmul(x, q, out=out), lambda: qmm.matmul_act(x, q, act="relu2", out=out),
+                 lambda: qmm.matmul(x, q, qmm.group_sums(x).cpu()), lambda: qmm.matmul(x, q, sk=2, reduce=False, part=torch.empty(2 * m * 256))]
+        for call in calls:
+            with pytest.raises(ValueError):
+                call()
+        pinned, want = torch.empty((m, 256), dtype=torch.bfloat16, pin_memory=True), qmm.matmul(x, q)
+        qmm.matmul(x, q, out=pinned)
+        torch.cuda.synchronize()
+        assert torch.equal(pinned, want.cpu())
